@@ -3,7 +3,8 @@
 What varies is how many queries one persistent warp carries at once (1..4: their list reads,
 visited checks and row copies overlap), how many warps share a block, how a round of vector rows
 is gathered (asynchronous copies of 4..16 rows into shared memory, or 1..2 rows per 8-lane group
-in registers) and whether the visited set starts in a shared-memory hash table. None of it changes
+in registers) and whether the visited set starts in a shared-memory hash table. The first candidate
+is the automatic shape, which also chooses between one warp and one block per query. None of it changes
 results (the GPU parity tests run every shape); all of it changes speed with the vector width, the
 beam size (efSearch, which sets the shared memory each query needs) and the batch size.
 ``autotune`` times the candidate shapes on the caller's own queries and leaves the fastest one set
@@ -19,6 +20,7 @@ from . import _capi
 
 # (warps_per_block, rows_per_group, visited_hash_log2, stage_rows, queries_per_warp, row_copy)
 DEFAULT_CANDIDATES = (
+    (0, 0, 0, 0, 0, 0),
     (4, 0, -1, 8, 1, 0), (2, 0, -1, 8, 1, 0), (4, 2, -1, -1, 1, 0),
     (4, 0, -1, 8, 2, 0), (4, 0, -1, 16, 2, 0), (2, 0, -1, 8, 2, 0), (4, 0, -1, 8, 2, 2),
     (4, 0, -1, 8, 3, 0), (4, 0, -1, 8, 4, 0), (4, 0, -1, 16, 4, 0), (2, 0, -1, 16, 4, 0), (4, 0, -1, 16, 4, 2),

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <numeric>
@@ -289,6 +290,55 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
   return NMSG_OK;
 }
 
+// Where the team kernel (one block per query, lists evaluated ahead) takes over from one warp per
+// query. Kernel time on B200, team against one-warp kernel, us:
+//   l2 1M x 128, efSearch 64:           1,200 queries 825 / 1,016   2,400: 1,012 / 1,043   4,000: 1,546 / 1,085
+//   l2sqr_sift 500K, efSearch 100:      1,000 queries 787 / 941     2,400: 1,188 / 944
+//   cosine 1M x 100, efSearch 200:      1,200 queries 1,353 / 2,355  2,400: 1,843 / 2,468  4,700: 3,052 / 2,838
+//   L1 200K x 100, efSearch 100:        1,200 queries 1,018 / 2,262  4,700: 2,156 / 2,430  10,000: 3,132 / 3,017
+//   negdot 200K x 960 with SearchOld queries: 2,000 queries 7,343 / 8,595   4,000: 13,791 / 15,869
+// so up to 8 queries per SM for the shapes with a lean or byte kernel, 16 for the other rows, 32 for
+// L1 / LInf (whose one-warp kernel holds one row per 8 lanes), and always where SearchOld runs (its
+// heaps sit in shared memory here).
+static int64_t team_limit(const DevIndex& d, const LaunchPlan& plan, int num_sms) {
+  if (plan.with_old) return INT64_MAX;
+  if (d.dist_type == kL1 || d.dist_type == kLInf) return 32 * num_sms;
+  if (plan.lean || d.dist_type == kSiftL2) return 8 * num_sms;
+  return 16 * num_sms;
+}
+
+TeamParams plan_team(const DevIndex& d, const nmsg_launch_config& cfg, const LaunchPlan& plan, int64_t nq,
+                     int num_sms) {
+  TeamParams t, none;
+  if (cfg.warps_per_block || cfg.rows_per_group || cfg.stage_rows || cfg.visited_hash_log2 || cfg.queries_per_warp ||
+      cfg.row_copy)
+    return none;  // an explicit shape of the one-warp kernels
+  if (nq > team_limit(d, plan, num_sms) || d.n >= (1 << 30)) return none;
+  // Eight warps and eight lists ahead while that many blocks are (nearly) resident, else four and four:
+  // 1,200 queries of l2 1M x 128 took 788-825 us with eight warps against 838 with four, 2,400 queries
+  // 1,142 against 1,012. SearchOld keeps eight (2,000 queries of the 960-wide mix: 7.3 against 8.3 ms).
+  const bool wide = plan.with_old || nq <= 8 * num_sms;
+  t.warps = wide ? 8 : 4;
+  t.spec = wide ? 8 : 4;
+  t.lcap = (d.maxM0 + 31) / 32 * 32;
+  t.mpad = std::max(32 * t.warps, (std::max(d.maxM, d.maxM0) + 31) / 32 * 32);
+  t.heap_items = plan.with_old ? 2048 : 0;
+  // The largest table with which every query is resident, down to 4,096 entries (2,048 for four
+  // warps): a long query that fills its table goes on with HBM reads (300 queries, efSearch 64: 598 us
+  // with 8,192 entries, 702 with 4,096), but resident queries come first (1,000: 893 against 802 us).
+  const int least = wide ? 12 : 11;
+  int bps = 0;
+  for (t.table_log2 = wide ? 14 : 11; t.table_log2 >= 10; --t.table_log2) {
+    t.l = team_layout(d.pitch, plan.region, t);
+    bps = 0;
+    if (t.l.total > kMaxSmemPerBlock || team_occupancy(d, t, plan.with_old, t.l.total, &bps) != 0) bps = 0;
+    if (bps >= 1 && (t.table_log2 <= least || (int64_t)bps * num_sms >= nq)) break;
+  }
+  if (bps < 1) return none;  // a beam that leaves no room for the table
+  t.blocks = (int)std::min<int64_t>(nq, (int64_t)bps * num_sms);
+  return t;
+}
+
 }  // namespace nmsg
 
 extern "C" {
@@ -554,9 +604,11 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   a.warp_smem = plan.warp_smem;
   const int gather = plan.gather, wpb = plan.wpb, bps = plan.blocks_per_sm;
   const int blocks = plain ? 0 : bps * h->num_sms;
-  const int slots = plain ? (h->cfg.plain_slots > 0 ? std::min(h->cfg.plain_slots, bps * h->num_sms)
-                                                   : bps * h->num_sms)
-                          : blocks * wpb * plan.ctx;
+  const int warp_slots = plain ? (h->cfg.plain_slots > 0 ? std::min(h->cfg.plain_slots, bps * h->num_sms)
+                                                        : bps * h->num_sms)
+                               : blocks * wpb * plan.ctx;
+  if (!plain) a.team = plan_team(d, h->cfg, plan, nq, h->num_sms);
+  const int slots = a.team.warps ? a.team.blocks : warp_slots;  // visited sets the batch needs
   a.ctx_per_warp = plan.ctx;
   a.bulk_rows = plan.bulk_rows ? 1 : 0;
   a.lean = plan.lean ? 1 : 0;
@@ -585,7 +637,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   a.visited_pitch = vpitch;
   a.epochs = h->epochs.as<uint8_t>();
   a.slot_locks = h->locks.as<int32_t>();
-  a.num_slots = slots;
+  a.num_slots = warp_slots;
   a.old_heap = h->old_heap.as<uint2>();
   a.old_heap_cap = h->old_cap;
   a.work_counter = h->counter.as<int32_t>();
@@ -595,7 +647,8 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   // several queries, and which queries start last decides when the batch ends). V1Merge batches of
   // one efSearch on the one-query-per-warp kernels.
   const bool split =
-      (plan.lean || (plan.ctx == 1 && !any_old)) && !plain && !ef_per_q && nq > slots && h->cfg.query_order != -1;
+      (plan.lean || (plan.ctx == 1 && !any_old)) && !plain && !ef_per_q && nq > warp_slots &&
+      h->cfg.query_order != -1;
   QueryParts parts;
   bool use_parts = false;
 

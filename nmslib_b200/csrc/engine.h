@@ -113,6 +113,38 @@ NMSG_HD inline int permuted_pos(int e, int dim) {
   return c * 32 + j * 2 + s;  // final half chunk of 16
 }
 
+constexpr int kTeamSlots = 16;  // evaluated lists a team search keeps at once
+constexpr int kTeamStateBytes = (20 + 9 * kTeamSlots) * 4;
+
+struct TeamLayout {  // byte offsets of a block's shared-memory pieces (its state comes first)
+  int q, items, tkey, tdist, merge, heap, tix, ste, work, total;
+};
+// Shape of a team search (search_team_kernel, team_kernel.cuh): one block per query.
+struct TeamParams {
+  int warps = 0;       // warps per block; 0: the team kernel is not used
+  int blocks = 0;      // grid
+  int table_log2 = 0;  // entries of the block's table of evaluated ids
+  int spec = 0;        // candidate lists evaluated per round, at most kTeamSlots
+  int lcap = 0;        // ids per evaluated list (maxM0 rounded up to 32)
+  int mpad = 0;        // entries of each merge scratch array: a list of any level, or one a thread
+  int heap_items = 0;  // SearchOld: candidate heap entries in shared memory
+  TeamLayout l{};
+};
+inline TeamLayout team_layout(int pitch, int region_items, const TeamParams& t) {
+  TeamLayout l;  // pitch is a multiple of 4, region_items even, mpad and lcap multiples of 32
+  l.q = kTeamStateBytes;
+  l.items = l.q + pitch * 4;
+  l.tkey = l.items + region_items * 8;
+  l.tdist = l.tkey + (4 << t.table_log2);
+  l.merge = l.tdist + (4 << t.table_log2);
+  l.heap = l.merge + t.mpad * 16;
+  l.tix = l.heap + t.heap_items * 8;
+  l.ste = l.tix + kTeamSlots * t.lcap * 2;
+  l.work = l.ste + 32 * t.warps * 2;
+  l.total = l.work + t.spec * t.lcap * 2;
+  return l;
+}
+
 struct SearchArgs {
   DevIndex ix;
   const float* queries = nullptr;   // [nq][dim]
@@ -156,6 +188,7 @@ struct SearchArgs {
   int bulk_rows = 0;                // search_multi_kernel: stage each row with one bulk copy (TMA
                                     // unit, mbarrier completion) instead of 16-byte copies per lane
   int lean = 0;                     // run search_lean_kernel (V1Merge, common index shapes)
+  TeamParams team;                  // team.warps > 0: search_team_kernel (level 0 only when split)
 };
 
 // Per-warp shared memory needed for the given caps.
@@ -178,6 +211,13 @@ NMSG_HD inline int lean_warp_smem_bytes(int dim, int region_items, int nbpad, in
 }
 int lean_occupancy(const DevIndex& ix, int warps_per_block, int smem_per_block, int* blocks_per_sm);
 int lean_smem_bytes(const DevIndex& ix, int region_items, int nbpad, int stage_rows);
+// The team kernel for an index (team_l2.cu, team_dot.cu, team_lp.cu, team_sift.cu), 4 or 8 warps per
+// block, with or without SearchOld.
+void* team_kernel_l2(const DevIndex& ix, int warps, bool with_old);
+void* team_kernel_dot(const DevIndex& ix, int warps, bool with_old);
+void* team_kernel_lp(const DevIndex& ix, int warps, bool with_old);
+void* team_kernel_sift(int warps, bool with_old);
+int team_occupancy(const DevIndex& ix, const TeamParams& t, bool with_old, int smem_per_block, int* blocks_per_sm);
 // Bytes one bulk row copy moves: the row rounded up to 16 bytes (the padding is zeros).
 NMSG_HD inline int bulk_row_bytes(const DevIndex& ix) { return ((ix.dim * 4 + 15) / 16) * 16; }
 

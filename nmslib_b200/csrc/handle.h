@@ -49,6 +49,11 @@ struct LaunchPlan {
 int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bool with_old, bool plain,
                 LaunchPlan* out, std::string* err);
 
+// The team kernel's shape for a batch of nq queries whose largest needs `region` items, or
+// warps == 0 when the batch runs on the kernels plan_launch chose (an explicit launch shape, or
+// no room in shared memory). region and nbpad are the plan's.
+TeamParams plan_team(const DevIndex& d, const nmsg_launch_config& cfg, const LaunchPlan& plan, int64_t nq, int num_sms);
+
 struct DeviceGuard {
   int prev = -1;
   explicit DeviceGuard(int dev) {

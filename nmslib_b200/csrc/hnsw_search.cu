@@ -862,7 +862,7 @@ __device__ void run_query(const SearchArgs& a, char* wsmem, int slot, int64_t qi
     curdist = __ldg(a.entry_dist + qi);
     w.st_dist = __ldg(a.entry_stats + 3 * qi + 0);
     w.st_greedy = __ldg(a.entry_stats + 3 * qi + 1);
-    w.st_bytes = __ldg(a.entry_stats + 3 * qi + 2);
+    w.st_bytes = (int64_t)ix.row_bytes * w.st_dist + 4LL * __ldg(a.entry_stats + 3 * qi + 2);
     if (cur < 0 || cur >= ix.n) {  // the descent pass gave up on this query
       search = false;
       w.failed = true;
@@ -875,7 +875,7 @@ __device__ void run_query(const SearchArgs& a, char* wsmem, int slot, int64_t qi
         a.entry_dist[qi] = curdist;
         a.entry_stats[3 * qi + 0] = w.st_dist;
         a.entry_stats[3 * qi + 1] = w.st_greedy;
-        a.entry_stats[3 * qi + 2] = (int32_t)w.st_bytes;
+        a.entry_stats[3 * qi + 2] = (int32_t)((w.st_bytes - (int64_t)ix.row_bytes * w.st_dist) / 4);
         const uint32_t key = ordered_key(curdist);
         atomicMin(a.entry_range + 0, key);
         atomicMax(a.entry_range + 1, key);
@@ -2003,6 +2003,20 @@ Kern lean_kernel_for(const DevIndex& ix) {
   return nullptr;
 }
 
+Kern team_kernel_for(const DevIndex& ix, int warps, bool with_old) {
+  void* k = nullptr;
+  switch (ix.dist_type) {
+    case kL2Sqr16Ext:
+    case kL2SqrExt: k = team_kernel_l2(ix, warps, with_old); break;
+    case kNormCosine:
+    case kNegDot: k = team_kernel_dot(ix, warps, with_old); break;
+    case kL1:
+    case kLInf: k = team_kernel_lp(ix, warps, with_old); break;
+    case kSiftL2: k = team_kernel_sift(warps, with_old); break;
+  }
+  return reinterpret_cast<Kern>(k);
+}
+
 Kern kernel_for(bool plain, int gather, bool with_old, int ctx = 1, int nch = 1) {
   if (ctx > 1 && !plain && !with_old && gather == 0) {
     if (ctx == 2) return nch == 1 ? search_multi_kernel<2, 1> : search_multi_kernel<2, 2>;
@@ -2079,8 +2093,22 @@ __global__ void __launch_bounds__(1024) order_by_entry_kernel(const float* __res
 
 }  // namespace
 
+namespace {
+int launch_team(const SearchArgs& a, bool with_old, cudaStream_t st) {
+  Kern kern = team_kernel_for(a.ix, a.team.warps, with_old);
+  if (!kern) return (int)cudaErrorInvalidDeviceFunction;
+  const int rc = allow_max_smem((const void*)kern);
+  if (rc != 0) return rc;
+  SearchArgs t = a;
+  t.num_slots = a.team.blocks;
+  kern<<<a.team.blocks, 32 * a.team.warps, a.team.l.total, st>>>(t);
+  return (int)cudaGetLastError();
+}
+}  // namespace
+
 int launch_search(const SearchArgs& a, bool plain, int gather, bool with_old, int blocks, int warps_per_block,
                   void* stream, const QueryParts* parts) {
+  if (!plain && a.team.warps && !a.entry_node) return launch_team(a, with_old, (cudaStream_t)stream);
   Kern kern = a.lean ? lean_kernel_for(a.ix) : kernel_for(plain, gather, with_old, a.ctx_per_warp, multi_list_chunks(a.ix));
   if (!kern) return (int)cudaErrorInvalidDeviceFunction;
   const int smem = a.warp_smem * (plain ? 1 : warps_per_block);
@@ -2122,6 +2150,7 @@ int launch_search(const SearchArgs& a, bool plain, int gather, bool with_old, in
     SearchArgs l = a;
     l.split = 2;
     l.order = a.entry_order;
+    if (a.team.warps) return launch_team(l, false, st);
     kern<<<blocks, 32 * warps_per_block, smem, st>>>(l);
     return (int)cudaGetLastError();
   }
@@ -2134,6 +2163,14 @@ int launch_search(const SearchArgs& a, bool plain, int gather, bool with_old, in
   else
     kern<<<blocks, 32 * warps_per_block, smem, (cudaStream_t)stream>>>(a);
   return (int)cudaGetLastError();
+}
+
+int team_occupancy(const DevIndex& ix, const TeamParams& t, bool with_old, int smem_per_block, int* blocks_per_sm) {
+  Kern kern = team_kernel_for(ix, t.warps, with_old);
+  if (!kern) return (int)cudaErrorInvalidDeviceFunction;
+  const int rc = allow_max_smem((const void*)kern);
+  if (rc != 0) return rc;
+  return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kern, 32 * t.warps, smem_per_block);
 }
 
 bool lean_supported(const DevIndex& ix) { return lean_kernel_for(ix) != nullptr; }

@@ -19,6 +19,11 @@ constexpr uint32_t kIdMask = 0x7fffffffu;
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ unsigned lanemask_lt() { return (1u << lane_id()) - 1u; }
+// A value every lane of the warp holds, as one the compiler knows to be uniform. Branches and loops
+// on such values keep the warp converged in its eyes; votes and shuffles under any other condition
+// are compiled to a collective sequence that costs around a hundred cycles each.
+__device__ __forceinline__ int uni(int x) { return __shfl_sync(kFull, x, 0); }
+__device__ __forceinline__ int warp_index() { return uni(threadIdx.x >> 5); }
 __device__ __forceinline__ float key_of(uint2 it) { return __uint_as_float(it.x); }
 __device__ __forceinline__ uint2 make_item(float key, int id, bool used) {
   return make_uint2(__float_as_uint(key), (uint32_t)id | (used ? kUsedBit : 0u));

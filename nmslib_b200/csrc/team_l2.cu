@@ -1,0 +1,19 @@
+// The team search kernels for squared L2 indices.
+#include "team_kernel.cuh"
+
+namespace nmsg {
+void* team_kernel_l2(const DevIndex& ix, int warps, bool with_old) {
+  if (with_old)
+    return warps == 4 ? (void*)search_team_kernel<kTeamL2, 0, 4, true> : (void*)search_team_kernel<kTeamL2, 0, 8, true>;
+  switch (ix.n16 >> 5) {
+    case 3:
+      return warps == 4 ? (void*)search_team_kernel<kTeamL2, 3, 4, false>
+                        : (void*)search_team_kernel<kTeamL2, 3, 8, false>;
+    case 4:
+      return warps == 4 ? (void*)search_team_kernel<kTeamL2, 4, 4, false>
+                        : (void*)search_team_kernel<kTeamL2, 4, 8, false>;
+  }
+  return warps == 4 ? (void*)search_team_kernel<kTeamL2, 0, 4, false>
+                    : (void*)search_team_kernel<kTeamL2, 0, 8, false>;
+}
+}  // namespace nmsg
