@@ -296,14 +296,13 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
 //   l2sqr_sift 500K, efSearch 100:      1,000 queries 787 / 941     2,400: 1,188 / 944
 //   cosine 1M x 100, efSearch 200:      1,200 queries 1,353 / 2,355  2,400: 1,843 / 2,468  4,700: 3,052 / 2,838
 //   L1 200K x 100, efSearch 100:        1,200 queries 1,018 / 2,262  4,700: 2,156 / 2,430  10,000: 3,132 / 3,017
-//   negdot 200K x 960 with SearchOld queries: 2,000 queries 7,343 / 8,595   4,000: 13,791 / 15,869
-// so up to 8 queries per SM for the shapes with a lean or byte kernel, 16 for the other rows, 32 for
-// L1 / LInf (whose one-warp kernel holds one row per 8 lanes), and always where SearchOld runs (its
-// heaps sit in shared memory here).
+//   negdot 200K x 960 with SearchOld queries: 300 queries 2,650 / 6,842   4,000: 8,463 / 15,869
+// so up to 8 queries per SM for bytes, 16 for float rows, 32 for L1 / LInf (whose one-warp kernel holds
+// one row per 8 lanes), and always where SearchOld runs (one lane works its heaps in the other kernels).
 static int64_t team_limit(const DevIndex& d, const LaunchPlan& plan, int num_sms) {
   if (plan.with_old) return INT64_MAX;
   if (d.dist_type == kL1 || d.dist_type == kLInf) return 32 * num_sms;
-  if (plan.lean || d.dist_type == kSiftL2) return 8 * num_sms;
+  if (d.dist_type == kSiftL2) return 8 * num_sms;
   return 16 * num_sms;
 }
 
@@ -322,7 +321,7 @@ TeamParams plan_team(const DevIndex& d, const nmsg_launch_config& cfg, const Lau
   t.spec = wide ? 8 : 4;
   t.lcap = (d.maxM0 + 31) / 32 * 32;
   t.mpad = std::max(32 * t.warps, (std::max(d.maxM, d.maxM0) + 31) / 32 * 32);
-  t.heap_items = plan.with_old ? 2048 : 0;
+  t.heap_items = plan.with_old ? 256 : 0;  // few queries need the heaps; room for a fourth block counts more
   // The largest table with which every query is resident, down to 4,096 entries (2,048 for four
   // warps): a long query that fills its table goes on with HBM reads (300 queries, efSearch 64: 598 us
   // with 8,192 entries, 702 with 4,096), but resident queries come first (1,000: 893 against 802 us).

@@ -114,7 +114,7 @@ NMSG_HD inline int permuted_pos(int e, int dim) {
 }
 
 constexpr int kTeamSlots = 16;  // evaluated lists a team search keeps at once
-constexpr int kTeamStateBytes = (20 + 9 * kTeamSlots) * 4;
+constexpr int kTeamStateBytes = (24 + 9 * kTeamSlots) * 4;
 
 struct TeamLayout {  // byte offsets of a block's shared-memory pieces (its state comes first)
   int q, items, tkey, tdist, merge, heap, tix, ste, work, total;

@@ -15,6 +15,7 @@
 // scope); per-request semantics are those of knnQueryBatch (python_bindings/nmslib.cc:142-168).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -80,6 +81,7 @@ struct nmsg_server {
   std::unordered_map<int64_t, Request> reqs;
   int64_t next_id = 1;
   int in_flight = 0;
+  int64_t in_flight_queries = 0, waiting_queries = 0;
   bool stop = false;
   std::thread worker;
   std::string worker_error;
@@ -107,8 +109,8 @@ struct nmsg_server {
     epochs.release();
   }
 
-  // Launch request r on lane li (worker thread, mu held).
-  int launch(int li, Request& r) {
+  // Launch request r on lane li (worker thread, mu held); load: queries in flight and waiting, r's too.
+  int launch(int li, Request& r, int64_t load) {
     Lane& l = lanes[li];
     const DevIndex& d = h->dev;
     const int dim = d.dim;
@@ -146,6 +148,10 @@ struct nmsg_server {
     a.warp_smem = plan.warp_smem;
     a.lean = plan.lean ? 1 : 0;
     a.bulk_rows = plan.bulk_rows ? 1 : 0;
+    // one block per query while the requests in flight and waiting leave the GPU room for it; a block
+    // takes one of the request's slots
+    a.team = plan_team(d, h->cfg, plan, load, h->num_sms);
+    if (a.team.warps) a.team.blocks = std::min(r.nq, l.nslots);
     const int wpb = plan.wpb;  // <= kWarpsPerBlock: the run holds whole blocks
     const int blocks = std::max(1, l.nslots / wpb);
     a.num_slots = blocks * wpb;
@@ -202,6 +208,7 @@ struct nmsg_server {
         l.req = -1;
         give_blocks(l.slot0 / kWarpsPerBlock, l.nslots / kWarpsPerBlock);
         --in_flight;
+        in_flight_queries -= r.nq;
         progressed = true;
       }
       if (progressed) cv_done.notify_all();
@@ -219,17 +226,20 @@ struct nmsg_server {
         const int b0 = take_blocks(need_blocks);
         if (b0 < 0) break;  // the oldest request waits for memory
         queue.pop_front();
+        waiting_queries -= r.nq;
         Lane& l = lanes[li];
         l.slot0 = b0 * kWarpsPerBlock;
         l.nslots = need_blocks * kWarpsPerBlock;
         ++in_flight;
-        const int rc = launch(li, r);
+        in_flight_queries += r.nq;
+        const int rc = launch(li, r, in_flight_queries + waiting_queries);
         if (rc != NMSG_OK) {
           r.status = rc;
           r.done = true;
           r.t_done = now_s();
           --in_flight;
           l.req = -1;
+          in_flight_queries -= r.nq;
           give_blocks(l.slot0 / kWarpsPerBlock, l.nslots / kWarpsPerBlock);
           cv_done.notify_all();
         }
@@ -341,6 +351,7 @@ NMSG_API int nmsg_server_submit(nmsg_server* s, const float* queries, int32_t nq
   r.t_arrival = t;
   *request_id = r.id;
   s->queue.push_back(r.id);
+  s->waiting_queries += nq;
   s->reqs.emplace(r.id, std::move(r));
   s->cv_work.notify_one();
   return NMSG_OK;

@@ -21,7 +21,8 @@ constexpr uint32_t kTabNew = 0x40000000u;      // and is kept by the expansions 
 constexpr uint32_t kTabIdMask = 0x3fffffffu;
 constexpr int kNoEntry = 0xffff;
 constexpr int kPlanFlush = -1;  // plans other than a number of lists: empty the table,
-constexpr int kPlanAgain = -2;  // or expand on (the front candidate's list is evaluated already)
+constexpr int kPlanAgain = -2;  // expand on (the front candidate's list is evaluated already),
+constexpr int kPlanRestart = -3;  // or search anew with heaps
 
 // What a block knows of its query between phases (shared memory; warp 0 writes).
 struct TeamState {
@@ -34,7 +35,10 @@ struct TeamState {
   int st_dist, st_expand, st_greedy, st_list_ints;
   int overflow;
   int line, ready;           // V1Merge: candidates in line (at most 16), how many of the first are evaluated
-  int pad;
+  int tied;                  // equal keys met where SearchOld's order among them would matter
+  float edge_in, edge_out;   // SearchOld's walk: the last key that stays in the array, the first that falls off,
+  float edge_tie;            // the key at the array's end that another like it fell off or was rejected at,
+  uint32_t late_tie;         // and the largest (ordered) key of an expanded candidate that had an equal beside it
   int kept, first;           // the expansions under way: kept neighbours, their smallest position
   int cnt[kTeamSlots];       // list lengths of the evaluated lists
   int slot_node[kTeamSlots]; // whose lists they are, or negative
@@ -82,6 +86,9 @@ struct TeamView {
   __device__ __forceinline__ int tlimit() const { return tsize() - tsize() / 5; }
 };
 
+// A distance as an integer of the same order, the two zeros as one.
+__device__ __forceinline__ uint32_t order_of(float d) { return ordered_key(__fadd_rn(d, 0.0f)); }
+
 // Finds or inserts id; *fresh is set when this call inserted it. The table always keeps free
 // entries (tlimit), so the probe ends.
 __device__ __forceinline__ int team_insert(const TeamView& v, uint32_t id, bool* fresh) {
@@ -120,16 +127,17 @@ template <int D>
 constexpr int team_group_lanes() {
   return D >= kTeamL1 ? 4 : 8;
 }
-// Rows one group holds in flight.
-template <int D>
+// Rows one group holds in flight: two where four warps' groups are fewer than a round's rows (about
+// 30), or a row is small; else one, with more of its pieces in flight.
+template <int D, int NF, int NW>
 constexpr int team_rows() {
-  return D == kTeamSift ? 4 : 2;
+  return D == kTeamSift || (D < kTeamL1 && NF > 0 && NW == 4) ? 2 : 1;
 }
 
 // Distances from the query to rows id[0..R) (act[r] false: not read, value meaningless), by the
 // lanes of a group; every lane of the warp calls it and every lane of the group gets the values.
-// Rows go from memory to registers, every 16-byte piece of up to four 32-float blocks in flight at
-// once. The arithmetic is combine() / lp_group_dist() / the l2sqr_sift branch of compute_dists()
+// Rows go from memory to registers, every 16-byte piece of up to four (wide rows: eight) 32-float
+// blocks in flight at once. The arithmetic is combine() / lp_group_dist() / the l2sqr_sift branch of compute_dists()
 // in hnsw_search.cu, order included:
 //  * l2, cosine, dot: lane j of 8 holds the reference's accumulator j (the permuted layout gives it
 //    its elements as one float4 per block); the 4-wide remainder and the scalar tail follow;
@@ -192,7 +200,7 @@ __device__ __forceinline__ void team_dists(const DevIndex& ix, const float* __re
           h1[r] = __ldg(reinterpret_cast<const float2*>(row[r] + nfull * 32) + 4 + a);
         }
       }
-      constexpr int U = 2;
+      constexpr int U = 4;
       for (int c0 = 0; c0 < nfull; c0 += U) {
         float4 x[R][U][2];
 #pragma unroll
@@ -287,7 +295,14 @@ __device__ __forceinline__ void team_dists(const DevIndex& ix, const float* __re
         h[r] = half && act[r] ? __ldg(reinterpret_cast<const float2*>(row[r] + nfull * 32) + j) : make_float2(0.f, 0.f);
         t[r] = tail && act[r] ? __ldg(reinterpret_cast<const float2*>(row[r] + ix.n16) + j) : make_float2(0.f, 0.f);
       }
-      constexpr int U = NF > 0 ? NF : 4;
+      constexpr int U = NF > 0 ? NF : 8;
+      if (NF == 0) {  // the rest of a wide row on its way to L2 while its first blocks are read
+        for (int c = U + j; c < nfull; c += 8) {
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (act[r]) prefetch_l2(row[r] + c * 32);
+        }
+      }
       for (int c0 = 0; c0 < nfull; c0 += U) {
         float4 x[R][U];
 #pragma unroll
@@ -363,7 +378,7 @@ __device__ __forceinline__ void team_dists(const DevIndex& ix, const float* __re
 // Distances of n rows by the whole block: row w's id is get(w), its distance goes to put(w, d).
 template <int D, int NF, int NW, class Get, class Put>
 __device__ __forceinline__ void team_eval(const DevIndex& ix, const float* q, int n, Get get, Put put) {
-  constexpr int GL = team_group_lanes<D>(), R = team_rows<D>(), kGroups = NW * 32 / GL;
+  constexpr int GL = team_group_lanes<D>(), R = team_rows<D, NF, NW>(), kGroups = NW * 32 / GL;
   const int group = threadIdx.x / GL;
   const int warp_first = warp_index() * (32 / GL);
   for (int base = 0; base + warp_first < n; base += kGroups * R) {
@@ -508,13 +523,14 @@ __device__ void team_result_offer(uint2* res, int& size, int k, float d, int nod
 // the batch merge when nothing ties, else std::sort's order and one insertion after another. Returns
 // the smallest insertion position; *num_io is the array's size.
 __device__ __noinline__ int team_insert_general(uint2* items, int* num_io, int cap, float* sk, int* sv, int qty,
-                                                float* tk, int* tv) {
+                                                float* tk, int* tv, int* tied) {
   const int lane = lane_id();
   int num = *num_io, p0 = 0x7fffffff;
   bool nan = false;
   for (int i = lane; i < qty; i += 32) nan |= !(sk[i] == sk[i]);
   nan = __any_sync(kFull, nan);  // no order to sort by: insert as they come
   if (nan || !merge_unsorted_batch(items, num, cap, sk, sv, qty, tk, tv, &p0)) {
+    if (lane == 0) *tied = 1;
     if (!nan) sort_like_std(sk, sv, qty, tk, tv);
     p0 = 0x7fffffff;
     for (int i = 0; i < qty; ++i) p0 = min(p0, sorted_insert(items, num, cap, sk[i], sv[i]));
@@ -568,6 +584,9 @@ __device__ __forceinline__ void team_plan(const SearchArgs& a, const TeamView& v
     st.ready = behind ? __ffs(behind) - 1 : 16;
     st.kept = 0;
     st.first = 0x7fffffff;
+    st.tied = 0;
+    st.edge_in = 0.0f;
+    st.edge_out = __int_as_float(0x7fffffff);  // NaN: equal to nothing
   }
 }
 
@@ -604,7 +623,7 @@ __device__ __forceinline__ void team_line_v1(const SearchArgs& a, const TeamView
     if (open && p < 16) {
       st.line_node[p] = (int)it.y;
       st.line_pos[p] = t;
-      st.line_key[p] = ordered_key(key_of(it));
+      st.line_key[p] = order_of(key_of(it));
     }
     found += __popc(m);
     if (!found) curr = min(t0 + 32, end);
@@ -616,6 +635,11 @@ __device__ __forceinline__ void team_line_v1(const SearchArgs& a, const TeamView
   }
   __syncwarp();
   team_plan(a, v, lane >= 16 ? st.slot_node[lane - 16] : -1, lane < found ? st.line_node[lane] : -1);
+  // over: SearchOld's walk, see team_expand_v1
+  if (lane == 0 && found == 0) {
+    const float last = key_of(items[st.num - 1]);
+    if (last == st.edge_tie || (st.num >= ef && order_of(last) <= st.late_tie)) st.plan = kPlanRestart;
+  }
 }
 
 // Warp 0: the kept neighbours of the expansions 0..n under way, inserted expansion after expansion in
@@ -649,7 +673,8 @@ __device__ __noinline__ void team_insert_ordered(const TeamView& v, int n, int e
       __syncwarp();
     }
     if (qty) {
-      const int p0 = team_insert_general(v.items(), &st.num, cap, v.sk(), v.sv(), qty, v.nb_d(), v.nb_id());
+      const int p0 = team_insert_general(v.items(), &st.num, cap, v.sk(), v.sv(), qty, v.nb_d(), v.nb_id(),
+                                         &st.tied);
       if (lane == 0) st.first = min(st.first, p0);
       __syncwarp();
     }
@@ -669,8 +694,20 @@ __device__ __noinline__ void team_insert_ordered(const TeamView& v, int n, int e
 // array item moves right by the number of kept keys not above it. Where that may not hold (equal
 // kept keys, two equal array keys, an equal one at the array's end, NaN, more kept than threads) the
 // kept ones are inserted one by one in the reference's order instead.
+//
+// `old`: SearchOld (hnsw_distfunc_opt.cc:285-381) with k <= ef, which is this walk too. Its candidates
+// leave the heap nearest first until one is past the closest set's largest, so the expanded ones are
+// the array's unused; its closest set is the best ef of everything, as the array is; its results are
+// the k first by (distance, node). Equal keys leave its heaps in an order of their own, which matters
+// in two places, and there the query is searched anew with heaps:
+//  * of two equal candidates the one expanded first may bring neighbours that cut the other off. Both
+//    are expanded in either order if the final largest lies past them (it only ever shrinks), and then
+//    all that either brings is seen; so the largest such key is held against the final largest;
+//  * where the array's end has one key of several equal ones, and the rest fell off or were rejected,
+//    SearchOld would still expand them if it came to them with that key as its largest: the walk must
+//    not expand a candidate of that key, nor end with it as the last.
 template <int NW>
-__device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamView& v, int k, int ef) {
+__device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamView& v, int k, int ef, bool old) {
   constexpr int kThreads = 32 * NW;
   const DevIndex& ix = a.ix;
   const int lane = lane_id(), warp = warp_index();
@@ -680,6 +717,7 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
   const int num = uni(st.num), ready = uni(st.ready);
   const float top_key = key_of(items[num - 1]);
   const bool open = num < ef;  // keep d < topKey || size < ef
+  const uint32_t edge = order_of(st.edge_tie);
   // ---- the nearest unvisited neighbour of every evaluated candidate at the front; a warp holds on to
   // the entries of its (first) list when they are one to a lane
   int my_cnt = 0, my_ti = kNoEntry;
@@ -693,7 +731,7 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
       const int ti = b + lane < cnt ? v.tix()[f * a.team.lcap + b + lane] : kNoEntry;
       const uint32_t key = ti != kNoEntry ? v.tkey()[ti] : kTabVisited;
       const float d = ti != kNoEntry ? v.tdist()[ti] : 0.0f;
-      if (!(key & kTabVisited)) near_key = min(near_key, ordered_key(d));
+      if (!(key & kTabVisited)) near_key = min(near_key, order_of(d));
       if (i == warp && cnt <= 32) {
         my_cnt = cnt;
         my_ti = ti;
@@ -718,6 +756,11 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
     const bool stop = lane > 0 && (lane >= ready || !(st.line_key[lane & 15] < least));
     n = __ffs(__ballot_sync(kFull, stop)) - 1;
     if (k > ef) n = 1;
+    if (old && __any_sync(kFull, lane < n && st.line_key[lane & 15] == edge)) {
+      __syncthreads();  // every warp has seen it
+      if (threadIdx.x == 0) st.plan = kPlanRestart;
+      return;
+    }
   }
   // ---- their lists: unvisited neighbours are marked, those that pass are kept
   for (int i = warp; i < n; i += NW) {
@@ -737,6 +780,7 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
       const bool pass = (d < top_key) || open;
       bool fresh = !(key & kTabVisited);  // of equal ids in one or several lists, one finds it unvisited
       if (fresh) fresh = !(atomicOr(v.tkey() + ti, pass ? kTabVisited | kTabNew : kTabVisited) & kTabVisited);
+      if (old && fresh && !pass && d == top_key) st.edge_tie = top_key;
       const unsigned km = __ballot_sync(kFull, fresh && pass);
       fresh_n += __popc(__ballot_sync(kFull, fresh));
       if (km) {
@@ -758,7 +802,9 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
       }
     }
     if (lane == 0) {
-      items[st.line_pos[i]].y = (uint32_t)st.line_node[i] | kUsedBit;
+      const int p = st.line_pos[i];
+      items[p].y = (uint32_t)st.line_node[i] | kUsedBit;
+      if (old && p + 1 < num && key_of(items[p + 1]) == key_of(items[p])) atomicMax(&st.late_tie, st.line_key[i]);
       atomicAdd(&st.st_dist, fresh_n);
       atomicAdd(&st.st_list_ints, 1 + cnt);
     }
@@ -792,11 +838,19 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
         rank += (s4.x < d) + (w + 1 < m && s4.y < d) + (w + 2 < m && s4.z < d) + (w + 3 < m && s4.w < d);
         equal += (s4.x == d) + (w + 1 < m && s4.y == d) + (w + 2 < m && s4.z == d) + (w + 3 < m && s4.w == d);
       }
-      const bool twin = lo < num && key_of(items[lo]) == d;
-      hard = equal != 1;  // itself; 0: NaN
-      hard |= twin && (lo + 1 >= num || lo + rank + 1 >= cap || key_of(items[lo + 1 < num ? lo + 1 : lo]) == d);
+      if (old && equal > 1)  // in the order they were kept
+        for (int w = 0; w < u; ++w) rank += sk[w] == d;
+      if (old) {
+        hard = equal == 0;  // NaN
+      } else {
+        const bool twin = lo < num && key_of(items[lo]) == d;
+        hard = equal != 1;  // itself; 0: NaN
+        hard |= twin && (lo + 1 >= num || lo + rank + 1 >= cap || key_of(items[lo + 1 < num ? lo + 1 : lo]) == d);
+      }
       pos = lo + rank;
       atomicMin(&st.first, lo);
+      if (old && pos == cap - 1) st.edge_in = d;
+      if (old && pos == cap) st.edge_out = d;
     }
     // the array in runs of one item a thread, from its tail: a run is read before it is written, and
     // what it writes lies below what the runs above it have moved
@@ -811,6 +865,8 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
           const float4 s4 = *reinterpret_cast<const float4*>(sk + w);
           c += (s4.x <= key) + (w + 1 < m && s4.y <= key) + (w + 2 < m && s4.z <= key) + (w + 3 < m && s4.w <= key);
         }
+        if (old && t + c == cap - 1) st.edge_in = key;
+        if (old && t + c == cap) st.edge_out = key;
       }
       if (top == num)
         general = __syncthreads_or(hard);
@@ -829,11 +885,22 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
   }
   if (general) {
     __syncthreads();
+    if (old && m <= kThreads) {
+      if (threadIdx.x == 0) st.plan = kPlanRestart;
+      return;
+    }
     if (threadIdx.x == 0) st.first = 0x7fffffff;
     __syncwarp();
     if (warp == 0) team_insert_ordered(v, n, ef, cap, a.team.lcap, st.line_slot);
   }
   __syncthreads();
+  if (old) {
+    if (uni(st.tied)) {
+      if (threadIdx.x == 0) st.plan = kPlanRestart;
+      return;
+    }
+    if (threadIdx.x == 0 && st.edge_in == st.edge_out) st.edge_tie = st.edge_in;
+  }
   if (warp == 0) {
     if (lane == 0) st.curr = min(st.line_pos[n - 1] + 1, st.first);  // everything before it is used
     __syncwarp();
@@ -1050,117 +1117,152 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
   }
   // ---- level 0: the entry point is visited and first in line
   const TeamHeap heap{v.heap(), OLD ? a.old_heap + (int64_t)slot * a.old_heap_cap : nullptr, a.team.heap_items};
-  if (warp == 0) {
-    if (lane == 0) {
-      bool fresh = false;
-      const int ti = team_insert(v, (uint32_t)cur, &fresh);
-      v.tkey()[ti] = (uint32_t)cur | kTabVisited;
-      st.curr = st.line = 0;
-      st.num = 1;
-      st.tcount = 1;
-      st.st_expand = 0;
-      st.overflow = 0;
-      if (!use_old) {
-        v.items()[0] = make_item(curdist, cur, false);
-      } else {
-        const uint2 e = make_uint2(__float_as_uint(curdist), (uint32_t)cur);
-        heap.set(0, make_uint2(__float_as_uint(-curdist), (uint32_t)cur));
-        v.items()[0] = v.items()[ef + 1] = e;
-        st.qsize = st.csize = st.rsize = 1;
-      }
-    }
-    if (lane < kTeamSlots) st.slot_node[lane] = -1;
-    __syncwarp();
-  }
+  // SearchOld with heaps, or (k <= ef, unless equal distances meet at the array's end) as V1Merge's walk
+  bool heaps = OLD && use_old && k > ef;
+  const int walk_dist = uni(st.st_dist), walk_ints = uni(st.st_list_ints);
+  bool restart = false;
   bool spilled = false;
   int epoch = 0;
   uint8_t* vis = a.visited + (int64_t)slot * a.visited_pitch;
-  if (warp == 0) {
-    if (use_old)
-      team_commit_old(a, v, heap, k, ef);
-    else
-      team_line_v1(a, v, ef);
-  }
   while (true) {
-    __syncthreads();
-    const int plan = uni(st.plan);
-    if (plan == 0) break;
-    if (plan == kPlanFlush) {
-      // the table is full: its visited ids move to the slot's epoch bytes in HBM, which every later
-      // insertion checks, and the lists evaluated ahead are dropped
-      if (!spilled) {
-        if (threadIdx.x == 0) st.epoch = a.epochs[slot] + 1;
-        __syncthreads();
-        epoch = st.epoch;
-        if (epoch == 256) {  // the byte wraps: clear (hnsw.h:582-589)
-          uint4* p = reinterpret_cast<uint4*>(vis);
-          for (int64_t t = threadIdx.x; t < a.visited_pitch / 16; t += NW * 32) p[t] = make_uint4(0, 0, 0, 0);
-          epoch = 1;
+    if (restart) {
+      for (int t = threadIdx.x; t < v.tsize() / 4; t += NW * 32)
+        reinterpret_cast<uint4*>(v.tkey())[t] = make_uint4(kTabEmpty, kTabEmpty, kTabEmpty, kTabEmpty);
+      heaps = true;
+      spilled = false;
+      __syncthreads();
+    }
+    if (warp == 0) {
+      if (lane == 0) {
+        bool fresh = false;
+        const int ti = team_insert(v, (uint32_t)cur, &fresh);
+        v.tkey()[ti] = (uint32_t)cur | kTabVisited;
+        st.curr = st.line = 0;
+        st.num = 1;
+        st.tcount = 1;
+        st.st_expand = 0;
+          st.overflow = 0;
+        st.edge_tie = __int_as_float(0x7fffffff);
+        st.late_tie = 0;
+        st.st_dist = walk_dist;
+        st.st_list_ints = walk_ints;
+        if (!heaps) {
+          v.items()[0] = make_item(curdist, cur, false);
+        } else {
+          const uint2 e = make_uint2(__float_as_uint(curdist), (uint32_t)cur);
+          heap.set(0, make_uint2(__float_as_uint(-curdist), (uint32_t)cur));
+          v.items()[0] = v.items()[ef + 1] = e;
+          st.qsize = st.csize = st.rsize = 1;
+        }
+      }
+      if (lane < kTeamSlots) st.slot_node[lane] = -1;
+      __syncwarp();
+    }
+    if (warp == 0) {
+      if (heaps)
+        team_commit_old(a, v, heap, k, ef);
+      else
+        team_line_v1(a, v, ef);
+    }
+    while (true) {
+      __syncthreads();
+      const int plan = uni(st.plan);
+      restart = OLD && plan == kPlanRestart;
+      if (plan == 0 || restart) break;
+      if (plan == kPlanFlush) {
+        // the table is full: its visited ids move to the slot's epoch bytes in HBM, which every later
+        // insertion checks, and the lists evaluated ahead are dropped
+        if (!spilled) {
+          if (threadIdx.x == 0) st.epoch = a.epochs[slot] + 1;
           __syncthreads();
+          epoch = st.epoch;
+          if (epoch == 256) {  // the byte wraps: clear (hnsw.h:582-589)
+            uint4* p = reinterpret_cast<uint4*>(vis);
+            for (int64_t t = threadIdx.x; t < a.visited_pitch / 16; t += NW * 32) p[t] = make_uint4(0, 0, 0, 0);
+            epoch = 1;
+            __syncthreads();
+          }
+          if (threadIdx.x == 0) a.epochs[slot] = (uint8_t)epoch;
+          spilled = true;
         }
-        if (threadIdx.x == 0) a.epochs[slot] = (uint8_t)epoch;
-        spilled = true;
-      }
-      for (int t = threadIdx.x; t < v.tsize(); t += NW * 32) {
-        const uint32_t key = v.tkey()[t];
-        if (key != kTabEmpty && (key & kTabVisited)) vis[key & kTabIdMask] = (uint8_t)epoch;
-        v.tkey()[t] = kTabEmpty;
-      }
-      if (threadIdx.x < kTeamSlots) st.slot_node[threadIdx.x] = -1;
-      if (threadIdx.x == 0) st.tcount = 0;
-      __syncthreads();
-      if (warp == 0) {
-        if (use_old)
-          team_commit_old(a, v, heap, k, ef);
-        else
-          team_line_v1(a, v, ef);
-      }
-      continue;
-    }
-    if (plan > 0) {
-      // ---- lists: one warp per candidate; ids not evaluated yet join the round's work
-      for (int i = warp; i < plan; i += NW) {
-        const int32_t* lst = ix.l0 + (int64_t)st.plan_node[i] * ix.l0_pitch;
-        const int f = uni(st.plan_slot[i]);
-        uint16_t* tix = v.tix() + f * a.team.lcap;
-        const int cnt = __ldg(lst);
-        for (int b = 0; b < ix.maxM0; b += 32) {
-          const int t = b + lane;
-          const int id = t < ix.maxM0 ? __ldg(lst + 1 + t) : 0;
-          bool valid = t < cnt;
-          if (spilled && valid) valid = vis[id] != (uint8_t)epoch;
-          bool fresh = false;
-          int ti = kNoEntry;
-          if (valid) ti = team_insert(v, (uint32_t)id, &fresh);
-          if (t < cnt) tix[t] = (uint16_t)ti;
-          const unsigned m = __ballot_sync(kFull, fresh);
-          int at = 0;
-          if (lane == 0 && m) at = atomicAdd(&st.work, __popc(m));
-          at = __shfl_sync(kFull, at, 0);
-          if (fresh) v.work()[at + __popc(m & lanemask_lt())] = (uint16_t)ti;
+        for (int t = threadIdx.x; t < v.tsize(); t += NW * 32) {
+          const uint32_t key = v.tkey()[t];
+          if (key != kTabEmpty && (key & kTabVisited)) vis[key & kTabIdMask] = (uint8_t)epoch;
+          v.tkey()[t] = kTabEmpty;
         }
-        if (lane == 0) st.cnt[f] = cnt;
+        if (threadIdx.x < kTeamSlots) st.slot_node[threadIdx.x] = -1;
+        if (threadIdx.x == 0) st.tcount = 0;
+        __syncthreads();
+        if (warp == 0) {
+          if (heaps)
+            team_commit_old(a, v, heap, k, ef);
+          else
+            team_line_v1(a, v, ef);
+        }
+        continue;
       }
-      __syncthreads();
-      // ---- rows
-      team_eval<D, NF, NW>(
-          ix, v.q(), uni(st.work), [&](int w) { return (int)(v.tkey()[v.work()[w]] & kTabIdMask); },
-          [&](int w, float d) { v.tdist()[v.work()[w]] = d; });
-      __syncthreads();
-      if (threadIdx.x == 0) st.tcount += st.work;
+      if (plan > 0) {
+        // ---- lists: one warp per candidate; ids not evaluated yet join the round's work
+        for (int i = warp; i < plan; i += NW) {
+          const int32_t* lst = ix.l0 + (int64_t)st.plan_node[i] * ix.l0_pitch;
+          const int f = uni(st.plan_slot[i]);
+          uint16_t* tix = v.tix() + f * a.team.lcap;
+          const int cnt = __ldg(lst);
+          for (int b = 0; b < ix.maxM0; b += 32) {
+            const int t = b + lane;
+            const int id = t < ix.maxM0 ? __ldg(lst + 1 + t) : 0;
+            bool valid = t < cnt;
+            if (spilled && valid) valid = vis[id] != (uint8_t)epoch;
+            bool fresh = false;
+            int ti = kNoEntry;
+            if (valid) ti = team_insert(v, (uint32_t)id, &fresh);
+            if (t < cnt) tix[t] = (uint16_t)ti;
+            const unsigned m = __ballot_sync(kFull, fresh);
+            int at = 0;
+            if (lane == 0 && m) at = atomicAdd(&st.work, __popc(m));
+            at = __shfl_sync(kFull, at, 0);
+            if (fresh) v.work()[at + __popc(m & lanemask_lt())] = (uint16_t)ti;
+          }
+          if (lane == 0) st.cnt[f] = cnt;
+        }
+        __syncthreads();
+        // ---- rows
+        team_eval<D, NF, NW>(
+            ix, v.q(), uni(st.work), [&](int w) { return (int)(v.tkey()[v.work()[w]] & kTabIdMask); },
+            [&](int w, float d) { v.tdist()[v.work()[w]] = d; });
+        __syncthreads();
+        if (threadIdx.x == 0) st.tcount += st.work;
+      }
+      // ---- expansions, then the next round's lists
+      if (heaps) {
+        if (warp == 0) team_commit_old(a, v, heap, k, ef);
+      } else {
+        team_expand_v1<NW>(a, v, k, ef, OLD && use_old);
+      }
     }
-    // ---- expansions, then the next round's lists
-    if (use_old) {
-      if (warp == 0) team_commit_old(a, v, heap, k, ef);
-    } else {
-      team_expand_v1<NW>(a, v, k, ef);
-    }
+    if (!OLD || !restart) break;
   }
   if (warp == 0) {
-    if (use_old) {
+    if (heaps) {
       if (st.overflow) set_status(a.status, NMSG_ERR_CAPACITY);
       write_result_row(a, qi, v.items() + (ef + 1), st.overflow ? 0 : st.rsize, true);
     } else {
+      if (OLD && use_old && lane == 0 && k < st.num && key_of(v.items()[k - 1]) == key_of(v.items()[k])) {
+        // equal keys across the k-th place: the smallest nodes of the run come first
+        uint2* items = v.items();
+        const float key = key_of(items[k]);
+        int lo = k - 1, hi = k + 1;
+        while (lo > 0 && key_of(items[lo - 1]) == key) --lo;
+        while (hi < st.num && key_of(items[hi]) == key) ++hi;
+        for (int i = lo; i < k; ++i)
+          for (int j = k; j < hi; ++j)
+            if ((items[j].y & kIdMask) < (items[i].y & kIdMask)) {
+              const uint2 it = items[i];
+              items[i] = items[j];
+              items[j] = it;
+            }
+      }
+      __syncwarp();
       write_result_row(a, qi, v.items(), min(k, st.num), false);
     }
     if (a.stats && lane == 0) {
