@@ -608,7 +608,7 @@ struct RerankArgs {
   int32_t* out_count;          // [nq]
   float* tau;                  // [nq] BF16 threshold that every true top-k vector reaches
   uint8_t* needs;              // optional [nq]: 1 = some list overflowed
-  int32_t* found;              // optional [nq]: entries found over all lists
+  int32_t* summary;            // optional [2]: most entries found for a query (raised), queries that overflowed (added)
 };
 
 // (key, id) order of the result: larger key first, then smaller id.
@@ -853,7 +853,10 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
     a.out_count[q] = have;
     a.tau[q] = have == kk ? __fsub_rd(__fsub_rd(kth, eps), fabsf(kth) * 1.1920929e-7f) : -INFINITY;
     if (a.needs) a.needs[q] = s_over ? 1 : 0;
-    if (a.found) a.found[q] = s_found;
+    if (a.summary) {
+      atomicMax(a.summary, s_found);
+      if (s_over) atomicAdd(a.summary + 1, 1);
+    }
   }
 }
 
@@ -870,9 +873,10 @@ struct BruteForceState {
   int kp = 0;       // padded dim (multiple of 64, <= 4096)
   float max_xn = 0; // largest |x|^2 over the base (l2 bound)
   DevBuf x16, x32, xn, xn_hi, xn_lo, xt_max, dx_max;
-  DevBuf q32, q16, qn_hi, qn_lo, eps, cand_key, cand_id, cand_cnt, tau, needs, qact, coll_id, coll_key, coll_cnt, found;
-  DevBuf out_id, out_key, out_cnt, scr_id, scr_key, fin_id, fin_key, fin_cnt, status;
+  DevBuf q32, q16, qn_hi, qn_lo, eps, cand_key, cand_id, cand_cnt, tau, needs, qact, coll_id, coll_key, coll_cnt;
+  DevBuf out_id, out_key, out_cnt, scr_id, scr_key, fin_id, fin_key, fin_cnt;
   DevBuf h_q, h_ids, h_dists, h_counts;
+  DevBuf result;  // summary (4 words: most found, overflowed, status), then ids, distances, counts
   CUtensorMap tmx;
 };
 
@@ -880,8 +884,8 @@ void destroy_bruteforce(BruteForceState* s) {
   if (!s) return;
   for (DevBuf* b : {&s->x16, &s->x32, &s->xn, &s->xn_hi, &s->xn_lo, &s->xt_max, &s->dx_max, &s->q32, &s->q16, &s->qn_hi,
                     &s->qn_lo, &s->eps, &s->cand_key, &s->cand_id, &s->cand_cnt, &s->tau, &s->needs, &s->qact,
-                    &s->coll_id, &s->coll_key, &s->coll_cnt, &s->found, &s->out_id, &s->out_key, &s->out_cnt, &s->scr_id, &s->scr_key,
-                    &s->fin_id, &s->fin_key, &s->fin_cnt, &s->status, &s->h_q, &s->h_ids, &s->h_dists, &s->h_counts})
+                    &s->coll_id, &s->coll_key, &s->coll_cnt, &s->out_id, &s->out_key, &s->out_cnt, &s->scr_id, &s->scr_key,
+                    &s->fin_id, &s->fin_key, &s->fin_cnt, &s->h_q, &s->h_ids, &s->h_dists, &s->h_counts, &s->result})
     b->release();
   delete s;
 }
@@ -1281,8 +1285,12 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
   BF_CUDA(s->coll_id.ensure(c_lists * kCollectLen * 4, false), "cudaMalloc(collection)");
   BF_CUDA(s->coll_key.ensure(c_lists * kCollectLen * 4, false), "cudaMalloc(collection)");
   BF_CUDA(s->coll_cnt.ensure(c_lists * 4, false), "cudaMalloc(collection)");
-  BF_CUDA(s->found.ensure(nq * 4, false), "cudaMalloc");
-  BF_CUDA(s->status.ensure(4, true), "cudaMalloc");
+  // the results behind the summary in one block, so that one copy takes both to the host
+  const size_t obytes = (size_t)nq * kmax * 4;
+  const size_t r_ids = 16, r_dists = r_ids + obytes, r_counts = r_dists + obytes;
+  const size_t r_bytes = r_counts + (size_t)nq * 4;
+  BF_CUDA(s->result.ensure(dev_ptrs ? r_ids : r_bytes, false), "cudaMalloc(results)");
+  int32_t* summary = s->result.as<int32_t>();
   const float max_xn = s->max_xn;
   prep_query_kernel<<<(mpad + 7) / 8, 256, 0, st>>>(qin, (int)nq, dim, kp, mpad, cosine, l2, s->xt_max.as<unsigned>(),
                                                      s->dx_max.as<unsigned>(), max_xn * 1.0001f, s->q32.as<float>(),
@@ -1291,7 +1299,7 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
   BF_CUDA(cudaGetLastError(), "prepare queries");
   CUtensorMap tmq;
   if (!make_tmap(&tmq, s->q16.p, mpad, kp, BM)) return bf_fail(NMSG_ERR_DEVICE, tmap_error("queries", mpad, kp, s->q16.p));
-  BF_CUDA(cudaMemsetAsync(s->status.p, 0, 4, st), "reset status");
+  BF_CUDA(cudaMemsetAsync(summary, 0, 16, st), "reset summary");
 
   // 1. top-CAND BF16 candidates of the sample, exact rerank -> tau
   GemmArgs ga;
@@ -1315,7 +1323,7 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
   ga.list_cnt = s->cand_cnt.as<int32_t>();
   ga.tau = s->tau.as<float>();
   ga.q_active = s->qact.as<uint8_t>();
-  ga.status = s->status.as<int32_t>();
+  ga.status = summary + 2;
   const int smem = SmemLayout(kb, ga.stages, ga.stream_q).total + 1024;
   BF_CUDA((cudaError_t)allow_max_smem((const void*)bf16_scan_kernel<0>), "smem attribute");
   BF_CUDA((cudaError_t)allow_max_smem((const void*)bf16_scan_kernel<1>), "smem attribute");
@@ -1369,15 +1377,22 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
   rb.out_keys = s->fin_key.as<DF>();
   rb.out_count = s->fin_cnt.as<int32_t>();
   rb.needs = s->needs.as<uint8_t>();
-  rb.found = s->found.as<int32_t>();
+  rb.summary = summary;
   BF_CUDA(cudaMemsetAsync(s->qact.p, 1, mpad, st), "reset flags");
   int64_t max_collected = 0, rescanned = 0, overflow = 0;
-  std::vector<uint8_t> flags_h(nq);
-  std::vector<int32_t> cnt_h(nq);
-  int32_t dstatus = 0;
+  int32_t sum_h[4];
+  int32_t* o_ids = dev_ptrs ? ids : reinterpret_cast<int32_t*>(s->result.as<char>() + r_ids);
+  float* o_d = dev_ptrs ? dists : reinterpret_cast<float*>(s->result.as<char>() + r_dists);
+  int32_t* o_c = dev_ptrs ? counts : reinterpret_cast<int32_t*>(s->result.as<char>() + r_counts);
+  // host results through the page-locked block unless direct copies are asked for or it cannot be had
+  bool pinned = !dev_ptrs && h->cfg.host_copy == 0;
+  if (pinned && h->pin_out.ensure(r_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    pinned = false;
+  }
   constexpr int kScans = 4;
   for (int attempt = 0; attempt < kScans; ++attempt) {
-    BF_CUDA(cudaMemsetAsync(s->found.p, 0, nq * 4, st), "reset counts");
+    if (attempt) BF_CUDA(cudaMemsetAsync(summary + 1, 0, 4, st), "reset summary");
     BF_CUDA(cudaMemsetAsync(s->needs.p, 0, mpad, st), "reset flags");
     bf16_scan_kernel<1><<<std::min(q_blocks * n_chunks, h->num_sms), Roles<1>::kThreads, smem, st>>>(tmq, s->tmx,
                                                                                                    gb);
@@ -1385,43 +1400,40 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
     rb.only = attempt == 0 ? nullptr : s->qact.as<uint8_t>();  // the other queries keep their results
     rerank_kernel<<<(unsigned)nq, kRerankThreads, 0, st>>>(rb);
     BF_CUDA(cudaGetLastError(), "rerank");
-    BF_CUDA(cudaMemcpyAsync(flags_h.data(), s->needs.p, nq, cudaMemcpyDeviceToHost, st), "copy flags");
-    BF_CUDA(cudaMemcpyAsync(cnt_h.data(), s->found.p, nq * 4, cudaMemcpyDeviceToHost, st), "copy counts");
-    BF_CUDA(cudaMemcpyAsync(&dstatus, s->status.p, 4, cudaMemcpyDeviceToHost, st), "copy status");
-    BF_CUDA(cudaStreamSynchronize(st), "brute-force scan");
-    if (dstatus) return bf_fail(dstatus, "brute-force scan reported a device-side error");
-    overflow = 0;
-    for (int64_t i = 0; i < nq; ++i) {
-      max_collected = std::max<int64_t>(max_collected, cnt_h[i]);
-      overflow += flags_h[i];
+    // the results follow at once: an overflow, which writes them again, is rare, and waiting for the
+    // summary first cost a round trip and a pageable copy per array (333 queries: 140 of 530 us)
+    finish_kernel<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(
+        s->fin_id.as<int32_t>(), s->fin_key.as<DF>(), s->fin_cnt.as<int32_t>(), (int)nq, k, kmax, space,
+        s->qn_hi.as<float>(), s->qn_lo.as<float>(), h->dev.ext_id, o_ids, o_d, o_c);
+    BF_CUDA(cudaGetLastError(), "finish");
+    if (pinned) {
+      BF_CUDA(cudaMemcpyAsync(h->pin_out.p, s->result.p, r_bytes, cudaMemcpyDeviceToHost, st), "copy results");
+      BF_CUDA(cudaStreamSynchronize(st), "brute-force scan");
+      std::memcpy(sum_h, h->pin_out.p, 16);
+    } else {
+      BF_CUDA(cudaMemcpyAsync(sum_h, summary, 16, cudaMemcpyDeviceToHost, st), "copy summary");
+      BF_CUDA(cudaStreamSynchronize(st), "brute-force scan");
     }
+    if (sum_h[2]) return bf_fail(sum_h[2], "brute-force scan reported a device-side error");
+    max_collected = sum_h[0];
+    overflow = sum_h[1];
     if (!overflow || attempt + 1 == kScans) break;
     if (attempt == 0) rescanned = overflow;
     BF_CUDA(cudaMemcpyAsync(s->qact.p, s->needs.p, mpad, cudaMemcpyDeviceToDevice, st), "copy flags");
   }
 
   // outputs
-  int32_t* o_ids = ids;
-  float* o_d = dists;
-  int32_t* o_c = counts;
-  if (!dev_ptrs) {
-    BF_CUDA(s->h_ids.ensure((size_t)nq * kmax * 4, false), "cudaMalloc(staging)");
-    BF_CUDA(s->h_dists.ensure((size_t)nq * kmax * 4, false), "cudaMalloc(staging)");
-    BF_CUDA(s->h_counts.ensure(nq * 4, false), "cudaMalloc(staging)");
-    o_ids = s->h_ids.as<int32_t>();
-    o_d = s->h_dists.as<float>();
-    o_c = s->h_counts.as<int32_t>();
-  }
-  finish_kernel<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(
-      s->fin_id.as<int32_t>(), s->fin_key.as<DF>(), s->fin_cnt.as<int32_t>(), (int)nq, k, kmax, space,
-      s->qn_hi.as<float>(), s->qn_lo.as<float>(), h->dev.ext_id, o_ids, o_d, o_c);
-  BF_CUDA(cudaGetLastError(), "finish");
-  if (!dev_ptrs) {
-    const HostPiece down[3] = {{ids, o_ids, (size_t)nq * kmax * 4}, {dists, o_d, (size_t)nq * kmax * 4},
-                               {counts, o_c, (size_t)nq * 4}};
-    BF_CUDA(copy_to_host(h->pin_out, h->cfg.host_copy == 0, down, 3, st), "copy results");
-  } else {
-    BF_CUDA(cudaStreamSynchronize(st), "brute-force results");
+  if (pinned) {
+    const char* pin = h->pin_out.as<char>();
+    const HostPiece out[3] = {{ids, pin + r_ids, obytes}, {dists, pin + r_dists, obytes},
+                              {counts, pin + r_counts, (size_t)nq * 4}};
+    if (r_bytes >= kStageMinBytes)
+      host_copy(out, 3);
+    else
+      for (const HostPiece& o : out) std::memcpy(o.dst, o.src, o.bytes);
+  } else if (!dev_ptrs) {
+    const HostPiece down[3] = {{ids, o_ids, obytes}, {dists, o_d, obytes}, {counts, o_c, (size_t)nq * 4}};
+    BF_CUDA(copy_to_host(h->pin_out, false, down, 3, st), "copy results");
   }
   if (stats) {
     stats[0] = (int64_t)s_tiles * BN;  // sample rows (the last tile may be partial)

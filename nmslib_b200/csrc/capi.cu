@@ -462,7 +462,7 @@ void nmsg_index_free(nmsg_index* h) {
     destroy_bruteforce(h->bf);
     h->bf = nullptr;
     for (DevBuf* b : {&h->vecs, &h->norms, &h->l0, &h->up_off, &h->up_links, &h->ext_id, &h->visited, &h->epochs, &h->locks,
-                      &h->old_heap, &h->counter, &h->status, &h->order, &h->kq, &h->efq, &h->q_stage,
+                      &h->old_heap, &h->counter, &h->block, &h->order, &h->kq, &h->efq, &h->q_stage,
                       &h->ids_stage, &h->dists_stage, &h->counts_stage, &h->stats_stage, &h->entry})
       b->release();
     h->pin_in.release();
@@ -526,6 +526,50 @@ int nmsg_set_launch_config(nmsg_index* h, const nmsg_launch_config* cfg) {
 }  // extern "C"
 
 namespace {
+
+// Layout of a host call's block (knn_batch_impl): the inputs when they are few, then counter and status,
+// ids, distances, counts and stats; bytes == 0: the call copies array by array.
+struct CallBlock {
+  bool in = false;  // the inputs are part of it
+  size_t kq = 0, efq = 0, order = 0, ctl = 0, ids = 0, dists = 0, counts = 0, stats = 0, bytes = 0;
+};
+constexpr size_t kCallBlockBytes = 1 << 20;
+
+int plan_block(nmsg_index* h, CallBlock* b, int64_t nq, size_t row_bytes, int32_t kmax, bool k_per_q, bool ef_per_q,
+               bool stats) {
+  const size_t n = (size_t)nq;
+  if (n * (8 * (size_t)kmax + 36) >= kCallBlockBytes) return NMSG_OK;
+  size_t at = 0;
+  auto take = [&](size_t bytes) {
+    const size_t off = at;
+    at += (bytes + 15) & ~size_t(15);
+    return off;
+  };
+  CallBlock s;
+  s.in = n * (row_bytes + 12) < kCallBlockBytes;
+  if (s.in) {
+    take(n * row_bytes);
+    if (k_per_q) s.kq = take(n * 4);
+    if (ef_per_q) {
+      s.efq = take(n * 4);
+      s.order = take(n * 4);
+    }
+  }
+  s.ctl = take(8);
+  s.ids = take(n * kmax * 4);
+  s.dists = take(n * kmax * 4);
+  s.counts = take(n * 4);
+  if (stats) s.stats = take(n * 32);
+  if ((s.in && h->pin_in.ensure(s.ctl + 8) != cudaSuccess) || h->pin_out.ensure(at - s.ctl) != cudaSuccess) {
+    cudaGetLastError();  // no page-locked memory: copy directly
+    return NMSG_OK;
+  }
+  const cudaError_t e = h->block.ensure(at, false);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(call block)");
+  s.bytes = at;
+  *b = s;
+  return NMSG_OK;
+}
 
 // The batch search behind nmsg_knn_batch (float queries and distances) and nmsg_knn_batch_u8
 // (l2sqr_sift: uint8 queries, int distances).
@@ -630,8 +674,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
       h->old_cap = cap;
     }
   }
-  NMSG_CUDA(h->counter.ensure(4, true), "cudaMalloc(counter)");
-  NMSG_CUDA(h->status.ensure(4, true), "cudaMalloc(status)");
+  NMSG_CUDA(h->counter.ensure(8, true), "cudaMalloc(counter)");  // the work counter, then the status word
   a.visited = h->visited.as<uint8_t>();
   a.visited_pitch = vpitch;
   a.epochs = h->epochs.as<uint8_t>();
@@ -640,7 +683,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   a.old_heap = h->old_heap.as<uint2>();
   a.old_heap_cap = h->old_cap;
   a.work_counter = h->counter.as<int32_t>();
-  a.status = h->status.as<int32_t>();
+  a.status = a.work_counter + 1;
 
   // Split search: worth it once the batch outnumbers the resident warps (some warps then run
   // several queries, and which queries start last decides when the batch ends). V1Merge batches of
@@ -651,6 +694,16 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   QueryParts parts;
   bool use_parts = false;
 
+  // A host call of up to a megabyte of results has them in one block with the status word, which one
+  // copy takes back through page-locked memory; with up to a megabyte of inputs these lie before it,
+  // behind them a zeroed counter and status, and one copy brings them all. Array by array that was two
+  // memsets and a pageable copy of about 15 us each: one query over 10K x 128 198 -> 150 us per call.
+  CallBlock block;
+  if (!dev_ptrs && h->cfg.host_copy == 0) {
+    rc = plan_block(h, &block, nq, (size_t)dim * (u8 ? 1 : 4), kmax, k_per_q != nullptr, ef_per_q != nullptr,
+                    stats != nullptr);
+    if (rc != NMSG_OK) return rc;
+  }
   // inputs / outputs
   const size_t qbytes = (size_t)nq * dim * (u8 ? 1 : 4), obytes = (size_t)nq * kmax * 4;
   if (dev_ptrs) {
@@ -662,12 +715,37 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
     a.dists = dists;
     a.counts = counts;
     a.stats = stats;
+  } else if (block.bytes && block.in) {
+    char* dev = h->block.as<char>();
+    char* pin = h->pin_in.as<char>();
+    std::memcpy(pin, queries_v, qbytes);
+    if (u8)
+      a.queries_u8 = reinterpret_cast<uint8_t*>(dev);
+    else
+      a.queries = reinterpret_cast<float*>(dev);
+    if (k_per_q) {
+      std::memcpy(pin + block.kq, k_per_q, (size_t)nq * 4);
+      a.k_per_q = reinterpret_cast<int32_t*>(dev + block.kq);
+    }
+    if (ef_per_q) {
+      std::memcpy(pin + block.efq, ef_per_q, (size_t)nq * 4);
+      a.ef_per_q = reinterpret_cast<int32_t*>(dev + block.efq);
+      // most expensive queries first, so the persistent blocks finish together
+      int32_t* order = reinterpret_cast<int32_t*>(pin + block.order);
+      std::iota(order, order + nq, 0);
+      std::stable_sort(order, order + nq, [&](int32_t x, int32_t y) { return ef_per_q[x] > ef_per_q[y]; });
+      a.order = reinterpret_cast<int32_t*>(dev + block.order);
+    }
+    std::memset(pin + block.ctl, 0, 8);
+    NMSG_CUDA(cudaMemcpyAsync(dev, pin, block.ctl + 8, cudaMemcpyHostToDevice, st), "copy queries");
   } else {
     NMSG_CUDA(h->q_stage.ensure(qbytes, false), "cudaMalloc(query staging)");
-    NMSG_CUDA(h->ids_stage.ensure(obytes, false), "cudaMalloc(id staging)");
-    NMSG_CUDA(h->dists_stage.ensure(obytes, false), "cudaMalloc(distance staging)");
-    NMSG_CUDA(h->counts_stage.ensure((size_t)nq * 4, false), "cudaMalloc(count staging)");
-    if (stats) NMSG_CUDA(h->stats_stage.ensure((size_t)nq * 32, false), "cudaMalloc(stats staging)");
+    if (!block.bytes) {
+      NMSG_CUDA(h->ids_stage.ensure(obytes, false), "cudaMalloc(id staging)");
+      NMSG_CUDA(h->dists_stage.ensure(obytes, false), "cudaMalloc(distance staging)");
+      NMSG_CUDA(h->counts_stage.ensure((size_t)nq * 4, false), "cudaMalloc(count staging)");
+      if (stats) NMSG_CUDA(h->stats_stage.ensure((size_t)nq * 32, false), "cudaMalloc(stats staging)");
+    }
     HostPiece up[3];
     int nup = 0;
     up[nup++] = HostPiece{h->q_stage.p, queries_v, qbytes};
@@ -675,10 +753,12 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
       a.queries_u8 = h->q_stage.as<uint8_t>();
     else
       a.queries = h->q_stage.as<float>();
-    a.ids = h->ids_stage.as<int32_t>();
-    a.dists = h->dists_stage.as<float>();
-    a.counts = h->counts_stage.as<int32_t>();
-    a.stats = stats ? h->stats_stage.as<int64_t>() : nullptr;
+    if (!block.bytes) {
+      a.ids = h->ids_stage.as<int32_t>();
+      a.dists = h->dists_stage.as<float>();
+      a.counts = h->counts_stage.as<int32_t>();
+      a.stats = stats ? h->stats_stage.as<int64_t>() : nullptr;
+    }
     if (k_per_q) {
       NMSG_CUDA(h->kq.ensure((size_t)nq * 4, false), "cudaMalloc(k per query)");
       up[nup++] = HostPiece{h->kq.p, k_per_q, (size_t)nq * 4};
@@ -721,6 +801,15 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
       NMSG_CUDA(copy_to_device(h->pin_in, h->cfg.host_copy == 0, up, nup, st), "copy queries");
     }
   }
+  if (block.bytes) {
+    char* dev = h->block.as<char>();
+    a.work_counter = reinterpret_cast<int32_t*>(dev + block.ctl);
+    a.status = a.work_counter + 1;
+    a.ids = reinterpret_cast<int32_t*>(dev + block.ids);
+    a.dists = reinterpret_cast<float*>(dev + block.dists);
+    a.counts = reinterpret_cast<int32_t*>(dev + block.counts);
+    a.stats = stats ? reinterpret_cast<int64_t*>(dev + block.stats) : nullptr;
+  }
   a.nbpad = plan.nbpad;
   if (split) {
     const size_t words = (size_t)nq * 6 + 4;  // node, distance, 3 counts, order; range
@@ -748,8 +837,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
       if (!h->capture_stream) NMSG_CUDA(cudaStreamCreateWithFlags(&h->capture_stream, cudaStreamNonBlocking), "stream");
       cudaStream_t cs = h->capture_stream;
       NMSG_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "begin capture");
-      cudaMemsetAsync(a.work_counter, 0, 4, cs);
-      cudaMemsetAsync(a.status, 0, 4, cs);
+      cudaMemsetAsync(a.work_counter, 0, 8, cs);
       const int lrc = launch_search(a, plain, gather, any_old, blocks, wpb, cs);
       cudaGraph_t graph = nullptr;
       const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
@@ -771,13 +859,31 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
     h->last_launches = split_launches;
     return NMSG_OK;
   }
-  NMSG_CUDA(cudaMemsetAsync(a.work_counter, 0, 4, st), "reset counter");
-  NMSG_CUDA(cudaMemsetAsync(a.status, 0, 4, st), "reset status");
+  if (!block.in) NMSG_CUDA(cudaMemsetAsync(a.work_counter, 0, 8, st), "reset counter and status");
   rc = launch_search(a, plain, gather, any_old, blocks, wpb, stream, use_parts ? &parts : nullptr);
-  if (rc != 0) return cuda_fail((cudaError_t)rc, "search kernel launch");
+  if (rc != 0) {
+    if (block.in) cudaStreamSynchronize(st);  // its upload reads the page-locked block
+    return cuda_fail((cudaError_t)rc, "search kernel launch");
+  }
   h->last_launches = split_launches + (use_parts ? 1 : 0);
   if (dev_ptrs) return NMSG_OK;
   int32_t dstatus = 0;
+  if (block.bytes) {
+    const size_t r = block.bytes - block.ctl;
+    const char* pin = h->pin_out.as<char>() - block.ctl;
+    NMSG_CUDA(cudaMemcpyAsync(h->pin_out.p, a.work_counter, r, cudaMemcpyDeviceToHost, st), "copy results");
+    NMSG_CUDA(cudaStreamSynchronize(st), "search");
+    std::memcpy(&dstatus, pin + block.ctl + 4, 4);
+    const HostPiece out[4] = {{ids, pin + block.ids, obytes},
+                              {dists_v, pin + block.dists, obytes},
+                              {counts, pin + block.counts, (size_t)nq * 4},
+                              {stats, pin + block.stats, stats ? (size_t)nq * 32 : 0}};
+    for (const HostPiece& o : out)
+      if (o.bytes) std::memcpy(o.dst, o.src, o.bytes);
+    h->last_status = dstatus;
+    if (dstatus != 0) return fail(dstatus, "the search kernel reported a device-side error (status " + std::to_string(dstatus) + ")");
+    return NMSG_OK;
+  }
   const HostPiece down[5] = {{ids, a.ids, obytes},
                              {dists_v, a.dists, obytes},
                              {counts, a.counts, (size_t)nq * 4},

@@ -105,8 +105,9 @@ struct nmsg_index {
   nmsg::DevIndex dev;
   nmsg::DevBuf vecs, norms, l0, up_off, up_links, ext_id;
   // search scratch (grown on demand)
-  nmsg::DevBuf visited, epochs, locks, old_heap, counter, status, order, kq, efq;
+  nmsg::DevBuf visited, epochs, locks, old_heap, counter, order, kq, efq;
   nmsg::DevBuf entry;       // split lean search: entry nodes, distances, counts, key range, order
+  nmsg::DevBuf block;       // a host call's results, and its inputs when they are few
   nmsg::DevBuf q_stage, ids_stage, dists_stage, counts_stage, stats_stage;
   nmsg::PinBuf pin_in, pin_out;  // page-locked staging of pageable host buffers
   int slots = 0;            // slots covered by visited/epochs/locks
