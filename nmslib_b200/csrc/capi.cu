@@ -262,6 +262,11 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
     const int nbpad = std::max(32, ((std::max(d.maxM, d.maxM0) + 31) / 32) * 32);
     const bool bulk = cfg.row_copy != 1;
     int rows = p.stage_rows;
+    // An expansion brings 9-14 new rows: 12 a round take most in one, where 8 took two row latencies,
+    // and still leave 7 blocks per SM for rows of up to 512 bytes (10K queries, 1M x 128, efSearch 64:
+    // search kernels 1,577 us with 8 rows, 1,481 with 12, 1,477 with 16; at efSearch 256, where the
+    // larger beam array takes the room, 4 to 12 rows are within 1 %).
+    if (cfg.stage_rows == 0 && p.region <= 160 && d.dim <= 128) rows = 12;
     if (bulk) cap_bulk_round(d, &rows);
     const int ws = lean_smem_bytes(d, p.region, nbpad, rows);
     if (ws <= kMaxSmemPerBlock) {
