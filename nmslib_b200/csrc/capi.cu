@@ -264,9 +264,10 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
     int rows = p.stage_rows;
     // An expansion brings 9-14 new rows: 12 a round take most in one, where 8 took two row latencies,
     // and still leave 7 blocks per SM for rows of up to 512 bytes (10K queries, 1M x 128, efSearch 64:
-    // search kernels 1,577 us with 8 rows, 1,481 with 12, 1,477 with 16; at efSearch 256, where the
-    // larger beam array takes the room, 4 to 12 rows are within 1 %).
-    if (cfg.stage_rows == 0 && p.region <= 160 && d.dim <= 128) rows = 12;
+    // search kernels 1,577 us with 8 rows, 1,481 with 12, 1,477 with 16). Larger beam arrays take the
+    // room: 8 rows there (1M x 100 cosine, efSearch 200: 3,093 us against 3,349 with 4; 1M x 128,
+    // efSearch 256: 3,990 against 4,060); rows over 512 bytes keep 4 (205 floats: 4,416 against 4,761).
+    if (cfg.stage_rows == 0 && d.dim <= 128) rows = p.region <= 160 ? 12 : p.region <= 320 ? 8 : rows;
     if (bulk) cap_bulk_round(d, &rows);
     const int ws = lean_smem_bytes(d, p.region, nbpad, rows);
     if (ws <= kMaxSmemPerBlock) {
@@ -299,7 +300,7 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
 // query. Kernel time on B200, team against one-warp kernel, us:
 //   l2 1M x 128, efSearch 64:           1,200 queries 825 / 1,016   2,400: 1,012 / 1,043   4,000: 1,546 / 1,085
 //   l2sqr_sift 500K, efSearch 100:      1,000 queries 787 / 941     2,400: 1,188 / 944
-//   cosine 1M x 100, efSearch 200:      1,200 queries 1,353 / 2,355  2,400: 1,843 / 2,468  4,700: 3,052 / 2,838
+//   cosine 1M x 100, efSearch 200:      1,200 queries 1,353 / 2,355  2,400: 1,843 / 2,468 (4,000: 2,132 alone)
 //   L1 200K x 100, efSearch 100:        1,200 queries 1,018 / 2,262  4,700: 2,156 / 2,430  10,000: 3,132 / 3,017
 //   negdot 200K x 960 with SearchOld queries: 300 queries 2,650 / 6,842   4,000: 8,463 / 15,869
 // so up to 8 queries per SM for bytes, 16 for float rows, 32 for L1 / LInf (whose one-warp kernel holds

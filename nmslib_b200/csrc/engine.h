@@ -198,7 +198,8 @@ int warp_smem_bytes(const DevIndex& ix, int region_items, int nbpad, int hash_lo
 int multi_list_chunks(const DevIndex& ix);
 int multi_warp_smem_bytes(const DevIndex& ix, int region_items, int nbpad, int stage_rows, int ctx);
 // The lean one-query-per-warp kernel (V1Merge; l2 / cosine / negdot rows of 16, 48, 64, 96, 128 or
-// 256 floats; lists of up to 64 ids): whether it covers an index, its occupancy and its shared
+// 256 floats, or of 33-143 and 193-207 floats with a remainder past a multiple of 16; lists of up to 64
+// ids): whether it covers an index, its occupancy and its shared
 // memory per warp.
 bool lean_supported(const DevIndex& ix);
 // The lean kernel for an index of the matching distance (lean_l2.cu / lean_cos.cu /
@@ -207,7 +208,7 @@ void* lean_kernel_l2(const DevIndex& ix);
 void* lean_kernel_cos(const DevIndex& ix);
 void* lean_kernel_negdot(const DevIndex& ix);
 NMSG_HD inline int lean_warp_smem_bytes(int dim, int region_items, int nbpad, int stage_rows) {
-  return region_items * 8 + nbpad * 16 + stage_rows * dim * 4 + 16;  // + the row mbarrier
+  return region_items * 8 + nbpad * 16 + stage_rows * ((dim + 3) & ~3) * 4 + 16;  // + the row mbarrier
 }
 int lean_occupancy(const DevIndex& ix, int warps_per_block, int smem_per_block, int* blocks_per_sm);
 int lean_smem_bytes(const DevIndex& ix, int region_items, int nbpad, int stage_rows);

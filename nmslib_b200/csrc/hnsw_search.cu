@@ -1994,9 +1994,12 @@ Kern pick(bool plain, int gather) {
 
 // The lean kernel for this index shape, or null when it has none.
 Kern lean_kernel_for(const DevIndex& ix) {
-  if (ix.dim % 16 != 0 || std::max(ix.maxM, ix.maxM0) > 64) return nullptr;
+  if (std::max(ix.maxM, ix.maxM0) > 64) return nullptr;
   switch (ix.dist_type) {
-    case kL2Sqr16Ext: return reinterpret_cast<Kern>(lean_kernel_l2(ix));
+    case kL2Sqr16Ext:
+    case kL2SqrExt:  // the 16-wide reduction goes with lengths that are multiples of 16
+      if ((ix.dim % 16 == 0) != (ix.dist_type == kL2Sqr16Ext)) return nullptr;
+      return reinterpret_cast<Kern>(lean_kernel_l2(ix));
     case kNormCosine: return reinterpret_cast<Kern>(lean_kernel_cos(ix));
     case kNegDot: return reinterpret_cast<Kern>(lean_kernel_negdot(ix));
   }

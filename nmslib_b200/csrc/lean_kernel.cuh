@@ -17,11 +17,14 @@ namespace nmsg {
 namespace {
 
 // ------------------------------------------------------------------ lean single-query kernel
-// search_lean_kernel<NF, HALF, SP, NCH>: the persistent one-query-per-warp V1Merge search for the
+// search_lean_kernel<NF, HALF, SP, NCH, TAIL>: the persistent one-query-per-warp V1Merge search for the
 // common index shapes, written for few instructions per expansion: rows of 32 * NF (+ 16 when
 // HALF) floats, the distance code fixed at compile time (SP 0: L2Sqr16Ext, 1: NormCosine, 2:
 // NegativeDotProduct, all through the reference's 16-wide kernels since the length is a multiple
-// of 16), lists of up to 32 * NCH ids. The query sits in registers (lane j of an 8-lane group holds
+// of 16), lists of up to 32 * NCH ids; with TAIL, rows of 1 to 15 floats more, whose remainder goes
+// through lean_combine_tail (10,000 queries, 1M x 100 cosine, efSearch 200: 3,840 us on the general
+// kernel, 3,093 here; 300K x 100 l2, efSearch 64: 1,790 -> 1,250; x 50 dot: 1,454 -> 863; x 130, lists of
+// 64: 3,029 -> 2,606; bound like the rest by the chain list, visited bytes, rows, merge). The query sits in registers (lane j of an 8-lane group holds
 // the float4 pieces it multiplies), every new neighbour's row is fetched by the lane that holds it
 // with one bulk copy (TMA unit) into the warp's staging rows, and warp-uniform state stays in
 // registers. The steps, arithmetic and tie rules are those of run_query above (greedy descent
@@ -77,14 +80,51 @@ __device__ __forceinline__ float2 sub2_rn(float2 a, float2 b) {
   return d;
 }
 
-template <int NF, bool HALF>
+template <int NF, bool HALF, bool TAIL>
 struct LeanQuery {
   float4 c[NF > 0 ? NF : 1];
   float2 h;
+  float t4[TAIL ? 3 : 1];  // elements [n16, n4): lane j < 4 has every 4th
+  float t1[TAIL ? 3 : 1];  // elements [n4, dim)
 };
 
-template <int NF, bool HALF, int SP>
-__device__ __forceinline__ float lean_row_dist(const LeanQuery<NF, HALF>& q, const float* __restrict__ row) {
+// Floats of one staged row: the row rounded up to 16 bytes (rows are zero-padded in memory).
+template <int NF, bool HALF, bool TAIL>
+__device__ __forceinline__ int lean_row_floats(const DevIndex& ix) {
+  return TAIL ? (ix.dim + 3) & ~3 : NF * 32 + (HALF ? 16 : 0);
+}
+
+// The reduction for rows with a remainder (length not a multiple of 16): the 8 accumulators folded to
+// 4, the 4-wide fused remainder, the sum, the scalar fused tail (impl_inline.h:100-121, 152-173).
+template <int SP, bool HALF, int NF>
+__device__ __forceinline__ float lean_combine_tail(const DevIndex& ix, const LeanQuery<NF, HALF, true>& q,
+                                                   const float* __restrict__ row, float acc) {
+  constexpr int n16 = NF * 32 + (HALF ? 16 : 0);
+  const int gb = lane_id() & ~7, j = lane_id() & 7;
+  float t4 = __fadd_rn(acc, __shfl_down_sync(kFull, acc, 4, 8));
+  const int n4 = ix.dim & ~3;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (n16 + 4 * i < n4) t4 = lean_term<SP>(q.t4[i], row[n16 + 4 * i + (j & 3)], t4);
+  float s = __fadd_rn(__shfl_sync(kFull, t4, gb), __shfl_sync(kFull, t4, gb + 1));
+  s = __fadd_rn(s, __shfl_sync(kFull, t4, gb + 2));
+  s = __fadd_rn(s, __shfl_sync(kFull, t4, gb + 3));
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (n4 + i < ix.dim) s = lean_term<SP>(q.t1[i], row[n4 + i], s);
+  if constexpr (SP == 1) {
+    const float mn = (s < 1.0f) ? s : 1.0f;
+    const float mx = (-1.0f < mn) ? mn : -1.0f;
+    const float v = __fsub_rn(1.0f, mx);
+    return (0.0f < v) ? v : 0.0f;
+  } else {
+    return SP == 2 ? -s : s;
+  }
+}
+
+template <int NF, bool HALF, int SP, bool TAIL>
+__device__ __forceinline__ float lean_row_dist(const DevIndex& ix, const LeanQuery<NF, HALF, TAIL>& q,
+                                               const float* __restrict__ row) {
   const int j = lane_id() & 7;
   float acc = 0.0f;
 #pragma unroll
@@ -115,7 +155,10 @@ __device__ __forceinline__ float lean_row_dist(const LeanQuery<NF, HALF>& q, con
       acc = lean_term<SP>(q.h.y, x.y, acc);
     }
   }
-  return lean_combine<SP>(acc);
+  if constexpr (TAIL)
+    return lean_combine_tail<SP, HALF, NF>(ix, q, row, acc);
+  else
+    return lean_combine<SP>(acc);
 }
 
 struct LeanWarp {  // a warp's shared-memory pieces and counters
@@ -138,11 +181,11 @@ struct LeanWarp {  // a warp's shared-memory pieces and counters
 // stage_rows: with w.bulk each row is one bulk copy issued by the lane that holds it, completing on
 // the warp's mbarrier; otherwise the round's ids are posted in w.sv and every lane copies 16-byte
 // pieces of the round's rows. Returns false if bulk copies did not complete within the wait bound.
-template <int NF, bool HALF, int SP, int NCH>
-__device__ bool lean_rows(const DevIndex& ix, LeanWarp& w, const LeanQuery<NF, HALF>& q, const bool (&has)[NCH],
+template <int NF, bool HALF, int SP, int NCH, bool TAIL>
+__device__ bool lean_rows(const DevIndex& ix, LeanWarp& w, const LeanQuery<NF, HALF, TAIL>& q, const bool (&has)[NCH],
                           const int (&pos)[NCH], const int (&id)[NCH], int nrows) {
-  constexpr int kDim = NF * 32 + (HALF ? 16 : 0);
-  constexpr uint32_t kRowBytes = kDim * 4;
+  const int kDim = lean_row_floats<NF, HALF, TAIL>(ix);
+  const uint32_t kRowBytes = kDim * 4;
   const int lane = lane_id(), g = lane >> 3;
   for (int base = 0; base < nrows; base += w.stage_rows) {
     const int rows = min(w.stage_rows, nrows - base);
@@ -164,7 +207,7 @@ __device__ bool lean_rows(const DevIndex& ix, LeanWarp& w, const LeanQuery<NF, H
         return false;
       }
     } else {
-      constexpr int kPieces = kRowBytes / 16;  // 16-byte pieces per row
+      const int kPieces = (int)kRowBytes / 16;  // 16-byte pieces per row
 #pragma unroll
       for (int h = 0; h < NCH; ++h)
         if (has[h] && pos[h] >= base && pos[h] < base + rows) w.sv[pos[h] - base] = id[h];
@@ -179,7 +222,7 @@ __device__ bool lean_rows(const DevIndex& ix, LeanWarp& w, const LeanQuery<NF, H
     for (int r0 = 0; r0 < rows; r0 += 4) {
       const int r = r0 + g;
       const bool act = r < rows;
-      const float d = lean_row_dist<NF, HALF, SP>(q, w.stage + (act ? r : 0) * kDim);
+      const float d = lean_row_dist<NF, HALF, SP, TAIL>(ix, q, w.stage + (act ? r : 0) * kDim);
       if (act && (lane & 7) == 0) w.nb_d[base + r] = d;
     }
     __syncwarp();
@@ -231,10 +274,10 @@ __device__ __forceinline__ bool lean_merge64(uint2* items, int& num, int cap, fl
 // Query qi in registers: lane j of each 8-lane group takes elements {32c + j + 8s} (s = 0..3) of
 // every 32-element block c — the permuted order of the stored rows — and, with HALF, elements
 // {32 NF + j + 8s} (s = 0, 1); a cosine query is normalised first as hnsw.h:486-497 does.
-template <int NF, bool HALF, int SP>
-__device__ LeanQuery<NF, HALF> lean_load_query(const SearchArgs& a, int64_t qi) {
+template <int NF, bool HALF, int SP, bool TAIL>
+__device__ LeanQuery<NF, HALF, TAIL> lean_load_query(const SearchArgs& a, int64_t qi) {
   const int lane = lane_id(), j = lane & 7;
-  constexpr int kDim = NF * 32 + (HALF ? 16 : 0);
+  const int kDim = TAIL ? a.ix.dim : NF * 32 + (HALF ? 16 : 0);
   const float* src = a.queries + qi * kDim;
   float s = 1.0f;
   bool scale = false;
@@ -257,19 +300,28 @@ __device__ LeanQuery<NF, HALF> lean_load_query(const SearchArgs& a, int64_t qi) 
     const float v = __ldg(src + e);
     return scale ? __fmul_rn(v, s) : v;
   };
-  LeanQuery<NF, HALF> q;
+  LeanQuery<NF, HALF, TAIL> q;
 #pragma unroll
   for (int c = 0; c < NF; ++c)
     q.c[c] = make_float4(ld(32 * c + j), ld(32 * c + j + 8), ld(32 * c + j + 16), ld(32 * c + j + 24));
   if constexpr (HALF) q.h = make_float2(ld(32 * NF + j), ld(32 * NF + j + 8));
+  if constexpr (TAIL) {
+    constexpr int n16 = NF * 32 + (HALF ? 16 : 0);
+    const int n4 = kDim & ~3;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      q.t4[i] = n16 + 4 * i < n4 ? ld(n16 + 4 * i + (j & 3)) : 0.0f;
+      q.t1[i] = n4 + i < kDim ? ld(n4 + i) : 0.0f;
+    }
+  }
   return q;
 }
 
-template <int NF, bool HALF, int SP, int NCH>
+template <int NF, bool HALF, int SP, int NCH, bool TAIL>
 __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t epoch) {
   const DevIndex& ix = a.ix;
   const int lane = lane_id();
-  const LeanQuery<NF, HALF> q = lean_load_query<NF, HALF, SP>(a, qi);
+  const LeanQuery<NF, HALF, TAIL> q = lean_load_query<NF, HALF, SP, TAIL>(a, qi);
   const int k = a.k_per_q ? a.k_per_q[qi] : a.k_default;
   const int ef = a.ef_per_q ? a.ef_per_q[qi] : a.ef_default;
   w.st_dist = w.st_expand = w.st_greedy = w.st_list_ints = 0;
@@ -295,7 +347,7 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
       pos[h] = 0;
       id[h] = cur;
     }
-    if (!lean_rows<NF, HALF, SP, NCH>(ix, w, q, has, pos, id, 1)) return false;
+    if (!lean_rows<NF, HALF, SP, NCH, TAIL>(ix, w, q, has, pos, id, 1)) return false;
     curdist = w.nb_d[0];
     w.st_dist += 1;
     for (int lev = ix.maxlevel; lev > 0; --lev) {
@@ -309,7 +361,7 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
           pos[h] = t;
           id[h] = has[h] ? __ldg(lst + 1 + t) : 0;
         }
-        if (!lean_rows<NF, HALF, SP, NCH>(ix, w, q, has, pos, id, cnt)) return false;
+        if (!lean_rows<NF, HALF, SP, NCH, TAIL>(ix, w, q, has, pos, id, cnt)) return false;
         w.st_greedy += 1;
         w.st_dist += cnt;
         w.st_list_ints += 1 + cnt;
@@ -408,7 +460,7 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
     w.st_expand += 1;
     w.st_list_ints += 1 + cnt;
     w.st_dist += nnew;
-    if (!lean_rows<NF, HALF, SP, NCH>(ix, w, q, has, pos, id, nnew)) return false;
+    if (!lean_rows<NF, HALF, SP, NCH, TAIL>(ix, w, q, has, pos, id, nnew)) return false;
     // keep d < topKey || size < ef (lists of up to 32 and arrays of up to 64: merged in registers
     // unless keys tie)
     bool merged = false;
@@ -482,10 +534,10 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
   return true;
 }
 
-template <int NF, bool HALF, int SP, int NCH>
+template <int NF, bool HALF, int SP, int NCH, bool TAIL = false>
 __global__ void __launch_bounds__(128, 8) search_lean_kernel(SearchArgs a) {
   extern __shared__ __align__(16) char smem[];
-  constexpr int kDim = NF * 32 + (HALF ? 16 : 0);
+  const int kDim = lean_row_floats<NF, HALF, TAIL>(a.ix);
   const int warp = threadIdx.x >> 5, lane = lane_id();
   char* ws = smem + warp * a.warp_smem;
   const int slot = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -528,17 +580,35 @@ __global__ void __launch_bounds__(128, 8) search_lean_kernel(SearchArgs a) {
       }
       if (lane == 0) a.epochs[slot] = (uint8_t)ep;
     }
-    if (!lean_query<NF, HALF, SP, NCH>(a, w, qi, (uint8_t)ep)) {
+    if (!lean_query<NF, HALF, SP, NCH, TAIL>(a, w, qi, (uint8_t)ep)) {
       if (lane == 0) set_status(a.status, NMSG_ERR_TIMEOUT);
       return;
     }
   }
 }
 
+template <int NF, bool HALF, int SP>
+void* lean_tail(bool two) {
+  return two ? (void*)search_lean_kernel<NF, HALF, SP, 2, true> : (void*)search_lean_kernel<NF, HALF, SP, 1, true>;
+}
+
 // The instantiation for this index's row length and list length (SP fixed by the file), or null.
 template <int SP>
 void* lean_kernel_select(const DevIndex& ix) {
   const bool two = std::max(ix.maxM, ix.maxM0) > 32;
+  if (ix.dim % 16) {
+    switch (ix.n16) {
+      case 32: return lean_tail<1, false, SP>(two);
+      case 48: return lean_tail<1, true, SP>(two);
+      case 64: return lean_tail<2, false, SP>(two);
+      case 80: return lean_tail<2, true, SP>(two);
+      case 96: return lean_tail<3, false, SP>(two);
+      case 112: return lean_tail<3, true, SP>(two);
+      case 128: return lean_tail<4, false, SP>(two);
+      case 192: return lean_tail<6, false, SP>(two);
+    }
+    return nullptr;
+  }
   switch (ix.dim) {
     case 16: return two ? (void*)search_lean_kernel<0, true, SP, 2> : (void*)search_lean_kernel<0, true, SP, 1>;
     case 48: return two ? (void*)search_lean_kernel<1, true, SP, 2> : (void*)search_lean_kernel<1, true, SP, 1>;
