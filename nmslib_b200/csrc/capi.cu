@@ -340,7 +340,8 @@ TeamParams plan_team(const DevIndex& d, const nmsg_launch_config& cfg, const Lau
     if (bps >= 1 && (t.table_log2 <= least || (int64_t)bps * num_sms >= nq)) break;
   }
   if (bps < 1) return none;  // a beam that leaves no room for the table
-  t.blocks = (int)std::min<int64_t>(nq, (int64_t)bps * num_sms);
+  t.resident = bps * num_sms;
+  t.blocks = (int)std::min<int64_t>(nq, t.resident);
   return t;
 }
 
@@ -657,7 +658,8 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
                                                         : bps * h->num_sms)
                                : blocks * wpb * plan.ctx;
   if (!plain) a.team = plan_team(d, h->cfg, plan, nq, h->num_sms);
-  const int slots = a.team.warps ? a.team.blocks : warp_slots;  // visited sets the batch needs
+  // visited sets: as many as the shape can have resident, so that batches of growing size do not grow them
+  const int slots = a.team.warps ? a.team.resident : warp_slots;
   a.ctx_per_warp = plan.ctx;
   a.bulk_rows = plan.bulk_rows ? 1 : 0;
   a.lean = plan.lean ? 1 : 0;
@@ -876,14 +878,14 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   int32_t dstatus = 0;
   if (block.bytes) {
     const size_t r = block.bytes - block.ctl;
-    const char* pin = h->pin_out.as<char>() - block.ctl;
+    const char* pin = h->pin_out.as<char>();  // the block from ctl on
     NMSG_CUDA(cudaMemcpyAsync(h->pin_out.p, a.work_counter, r, cudaMemcpyDeviceToHost, st), "copy results");
     NMSG_CUDA(cudaStreamSynchronize(st), "search");
-    std::memcpy(&dstatus, pin + block.ctl + 4, 4);
-    const HostPiece out[4] = {{ids, pin + block.ids, obytes},
-                              {dists_v, pin + block.dists, obytes},
-                              {counts, pin + block.counts, (size_t)nq * 4},
-                              {stats, pin + block.stats, stats ? (size_t)nq * 32 : 0}};
+    std::memcpy(&dstatus, pin + 4, 4);
+    const HostPiece out[4] = {{ids, pin + (block.ids - block.ctl), obytes},
+                              {dists_v, pin + (block.dists - block.ctl), obytes},
+                              {counts, pin + (block.counts - block.ctl), (size_t)nq * 4},
+                              {stats, stats ? pin + (block.stats - block.ctl) : pin, stats ? (size_t)nq * 32 : 0}};
     for (const HostPiece& o : out)
       if (o.bytes) std::memcpy(o.dst, o.src, o.bytes);
     h->last_status = dstatus;

@@ -19,17 +19,18 @@ namespace {
 // ------------------------------------------------------------------ lean single-query kernel
 // search_lean_kernel<NF, HALF, SP, NCH, TAIL>: the persistent one-query-per-warp V1Merge search for the
 // common index shapes, written for few instructions per expansion: rows of 32 * NF (+ 16 when
-// HALF) floats, the distance code fixed at compile time (SP 0: L2Sqr16Ext, 1: NormCosine, 2:
-// NegativeDotProduct, all through the reference's 16-wide kernels since the length is a multiple
-// of 16), lists of up to 32 * NCH ids; with TAIL, rows of 1 to 15 floats more, whose remainder goes
-// through lean_combine_tail (10,000 queries, 1M x 100 cosine, efSearch 200: 3,840 us on the general
-// kernel, 3,093 here; 300K x 100 l2, efSearch 64: 1,790 -> 1,250; x 50 dot: 1,454 -> 863; x 130, lists of
-// 64: 3,029 -> 2,606; bound like the rest by the chain list, visited bytes, rows, merge). The query sits in registers (lane j of an 8-lane group holds
-// the float4 pieces it multiplies), every new neighbour's row is fetched by the lane that holds it
-// with one bulk copy (TMA unit) into the warp's staging rows, and warp-uniform state stays in
-// registers. The steps, arithmetic and tie rules are those of run_query above (greedy descent
-// hnsw_distfunc_opt.cc:168-198, SearchV1Merge :200-283, push_or_replace_non_empty_exp
-// sort_arr_bi.h:159-199), so results and per-query counts are identical to it bit for bit.
+// HALF) floats, the distance code fixed at compile time (SP 0: L2Sqr16Ext, or L2SqrExt with TAIL, 1:
+// NormCosine, 2: NegativeDotProduct, through the reference's 16-wide kernels), lists of up to 32 * NCH
+// ids; with TAIL, rows of 1 to 15 floats more, whose remainder goes through lean_combine_tail. The
+// query sits in registers (lane j of an 8-lane group holds the float4 pieces it multiplies), every new
+// neighbour's row is fetched by the lane that holds it with one bulk copy (TMA unit) into the warp's
+// staging rows, and warp-uniform state stays in registers. The steps, arithmetic and tie rules are
+// those of run_query in hnsw_search.cu (greedy descent hnsw_distfunc_opt.cc:168-198, SearchV1Merge
+// :200-283, push_or_replace_non_empty_exp sort_arr_bi.h:159-199), so results and per-query counts are
+// identical to it bit for bit.
+// TAIL, search kernels against the general kernel it replaces (10,000 queries): 1M x 100 cosine,
+// efSearch 200: 3,840 -> 3,093 us; 300K x 100 l2, efSearch 64: 1,790 -> 1,250; x 50 dot: 1,454 -> 863;
+// x 130 l2, lists of 64: 3,029 -> 2,606. Bound like the rest by the chain list, visited bytes, rows, merge.
 
 template <int SP>
 __device__ __forceinline__ float lean_term(float q, float x, float acc) {
