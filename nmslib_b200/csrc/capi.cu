@@ -262,12 +262,16 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
     const int nbpad = std::max(32, ((std::max(d.maxM, d.maxM0) + 31) / 32) * 32);
     const bool bulk = cfg.row_copy != 1;
     int rows = p.stage_rows;
-    // An expansion brings 9-14 new rows: 12 a round take most in one, where 8 took two row latencies,
-    // and still leave 7 blocks per SM for rows of up to 512 bytes (10K queries, 1M x 128, efSearch 64:
-    // search kernels 1,577 us with 8 rows, 1,481 with 12, 1,477 with 16). Larger beam arrays take the
-    // room: 8 rows there (1M x 100 cosine, efSearch 200: 3,093 us against 3,349 with 4; 1M x 128,
-    // efSearch 256: 3,990 against 4,060); rows over 512 bytes keep 4 (205 floats: 4,416 against 4,761).
-    if (cfg.stage_rows == 0 && d.dim <= 128) rows = p.region <= 160 ? 12 : p.region <= 320 ? 8 : rows;
+    // An expansion brings 9-14 new rows: 12 a round take most in one, where 8 take two row latencies
+    // (10K queries, search kernels, rows per round 4 / 8 / 12: 1M x 128, efSearch 100: 2,236 / 2,045 /
+    // 1,985 us) until the beam array or lists of more than 32 ids take the blocks' room (efSearch 128:
+    // 2,466 / 2,250 / 2,287, 320: 4,532 / 4,452 / 4,727; 1M x 100 with lists of 48, efSearch 32: 1,206 /
+    // 1,088 / 1,073, 100: 2,253 / 2,039 / 2,171, 200: 3,335 / 3,086 / 3,373, 256: 3,872 / 4,113 / 3,981).
+    // Rows over 512 bytes keep 8 up to efSearch 160, then 4 (205 floats, efSearch 200: 4,416 / 4,761).
+    if (cfg.stage_rows == 0 && d.dim <= 128) {
+      const bool short_lists = std::max(d.maxM, d.maxM0) <= 32;
+      rows = p.region <= (short_lists ? 112 : 64) ? 12 : p.region <= (short_lists ? 400 : 220) ? 8 : 4;
+    }
     if (bulk) cap_bulk_round(d, &rows);
     const int ws = lean_smem_bytes(d, p.region, nbpad, rows);
     if (ws <= kMaxSmemPerBlock) {
