@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include "engine.h"
@@ -607,8 +608,8 @@ __device__ __forceinline__ int team_peek(const SearchArgs& a, const TeamView& v,
 }
 
 // Warp 0, V1Merge: the line (the unused among the items that may be expanded, from the first on, up
-// to 16) and the next round's plan.
-__device__ __forceinline__ void team_line_v1(const SearchArgs& a, const TeamView& v, int ef) {
+// to 16) and the next round's plan. kth: SearchOld's walk, the length of its result; else past any array.
+__device__ __forceinline__ void team_line_v1(const SearchArgs& a, const TeamView& v, int ef, int kth) {
   const int lane = lane_id();
   TeamState& st = v.st();
   const uint2* items = v.items();
@@ -638,7 +639,9 @@ __device__ __forceinline__ void team_line_v1(const SearchArgs& a, const TeamView
   // over: SearchOld's walk, see team_expand_v1
   if (lane == 0 && found == 0) {
     const float last = key_of(items[st.num - 1]);
-    if (last == st.edge_tie || (st.num >= ef && order_of(last) <= st.late_tie)) st.plan = kPlanRestart;
+    if (last == st.edge_tie || (st.num >= ef && order_of(last) <= st.late_tie) ||
+        (kth < st.num && key_of(items[kth - 1]) == key_of(items[kth])))
+      st.plan = kPlanRestart;
   }
 }
 
@@ -698,14 +701,17 @@ __device__ __noinline__ void team_insert_ordered(const TeamView& v, int n, int e
 // `old`: SearchOld (hnsw_distfunc_opt.cc:285-381) with k <= ef, which is this walk too. Its candidates
 // leave the heap nearest first until one is past the closest set's largest, so the expanded ones are
 // the array's unused; its closest set is the best ef of everything, as the array is; its results are
-// the k first by (distance, node). Equal keys leave its heaps in an order of their own, which matters
-// in two places, and there the query is searched anew with heaps:
+// the k nearest of them. Equal keys leave its heaps in an order of their own, which matters in three
+// places, and there the query is searched anew with heaps:
 //  * of two equal candidates the one expanded first may bring neighbours that cut the other off. Both
 //    are expanded in either order if the final largest lies past them (it only ever shrinks), and then
 //    all that either brings is seen; so the largest such key is held against the final largest;
 //  * where the array's end has one key of several equal ones, and the rest fell off or were rejected,
 //    SearchOld would still expand them if it came to them with that key as its largest: the walk must
-//    not expand a candidate of that key, nor end with it as the last.
+//    not expand a candidate of that key, nor end with it as the last;
+//  * a result queue that holds k rejects an equal distance whatever its node (knnqueue.h:55-64), so of
+//    equal keys on both sides of the k-th place those found first are the results, an order the array
+//    does not keep: the walk must not end with such a pair.
 template <int NW>
 __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamView& v, int k, int ef, bool old) {
   constexpr int kThreads = 32 * NW;
@@ -904,7 +910,7 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
   if (warp == 0) {
     if (lane == 0) st.curr = min(st.line_pos[n - 1] + 1, st.first);  // everything before it is used
     __syncwarp();
-    team_line_v1(a, v, ef);
+    team_line_v1(a, v, ef, old ? k : INT_MAX);
   }
 }
 
@@ -1119,6 +1125,7 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
   const TeamHeap heap{v.heap(), OLD ? a.old_heap + (int64_t)slot * a.old_heap_cap : nullptr, a.team.heap_items};
   // SearchOld with heaps, or (k <= ef, unless equal distances meet at the array's end) as V1Merge's walk
   bool heaps = OLD && use_old && k > ef;
+  const int kth = OLD && use_old ? k : INT_MAX;
   const int walk_dist = uni(st.st_dist), walk_ints = uni(st.st_list_ints);
   bool restart = false;
   bool spilled = false;
@@ -1141,7 +1148,7 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
         st.num = 1;
         st.tcount = 1;
         st.st_expand = 0;
-          st.overflow = 0;
+        st.overflow = 0;
         st.edge_tie = __int_as_float(0x7fffffff);
         st.late_tie = 0;
         st.st_dist = walk_dist;
@@ -1162,7 +1169,7 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
       if (heaps)
         team_commit_old(a, v, heap, k, ef);
       else
-        team_line_v1(a, v, ef);
+        team_line_v1(a, v, ef, kth);
     }
     while (true) {
       __syncthreads();
@@ -1197,7 +1204,7 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
           if (heaps)
             team_commit_old(a, v, heap, k, ef);
           else
-            team_line_v1(a, v, ef);
+            team_line_v1(a, v, ef, kth);
         }
         continue;
       }
@@ -1247,22 +1254,6 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
       if (st.overflow) set_status(a.status, NMSG_ERR_CAPACITY);
       write_result_row(a, qi, v.items() + (ef + 1), st.overflow ? 0 : st.rsize, true);
     } else {
-      if (OLD && use_old && lane == 0 && k < st.num && key_of(v.items()[k - 1]) == key_of(v.items()[k])) {
-        // equal keys across the k-th place: the smallest nodes of the run come first
-        uint2* items = v.items();
-        const float key = key_of(items[k]);
-        int lo = k - 1, hi = k + 1;
-        while (lo > 0 && key_of(items[lo - 1]) == key) --lo;
-        while (hi < st.num && key_of(items[hi]) == key) ++hi;
-        for (int i = lo; i < k; ++i)
-          for (int j = k; j < hi; ++j)
-            if ((items[j].y & kIdMask) < (items[i].y & kIdMask)) {
-              const uint2 it = items[i];
-              items[i] = items[j];
-              items[j] = it;
-            }
-      }
-      __syncwarp();
       write_result_row(a, qi, v.items(), min(k, st.num), false);
     }
     if (a.stats && lane == 0) {
