@@ -891,7 +891,8 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
   }
   if (general) {
     __syncthreads();
-    if (old && m <= kThreads) {
+    // the walk follows no ties here: neither those that made it general nor those among what falls off
+    if (old && (m <= kThreads || num + m > cap)) {
       if (threadIdx.x == 0) st.plan = kPlanRestart;
       return;
     }
