@@ -662,8 +662,9 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
                                                         : bps * h->num_sms)
                                : blocks * wpb * plan.ctx;
   if (!plain) a.team = plan_team(d, h->cfg, plan, nq, h->num_sms);
-  // visited sets: as many as the shape can have resident, so that batches of growing size do not grow them
-  const int slots = a.team.warps ? a.team.resident : warp_slots;
+  // visited sets: as many as any batch size can have resident at this beam size, so that batches of
+  // growing size do not grow them (an allocation in mid-service, refused under stream capture)
+  const int slots = std::max(warp_slots, a.team.resident);
   a.ctx_per_warp = plan.ctx;
   a.bulk_rows = plan.bulk_rows ? 1 : 0;
   a.lean = plan.lean ? 1 : 0;

@@ -67,7 +67,7 @@ struct DeviceGuard {
   }
 };
 
-// A grow-only device buffer.
+// A grow-only device buffer. With `zero` its bytes are zero on return, for work on any stream.
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -79,8 +79,10 @@ struct DevBuf {
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) return e;
     bytes = want;
-    if (zero) return cudaMemset(p, 0, want);
-    return cudaSuccess;
+    // a memset runs on the legacy stream, which callers' non-blocking streams do not wait for
+    if (zero) e = cudaMemset(p, 0, want);
+    if (zero && e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e;
   }
   void release() {
     if (p) cudaFree(p);
