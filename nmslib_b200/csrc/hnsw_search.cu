@@ -643,6 +643,8 @@ __device__ void search_v1merge(const SearchArgs& a, WarpCtx& w, int64_t qi, int 
   const int cap = max(ef, k);
   uint2* items = w.items;
   int num = 1;
+  constexpr bool kInt = R == kSiftGather;
+  if (!kInt && !(curdist == curdist)) w.st_greedy = ~w.st_greedy;  // see insert_batch
   if (lane == 0) items[0] = make_item(curdist, cur, false);
   visit_one(w, cur);
   int curr = 0;
@@ -690,18 +692,7 @@ __device__ void search_v1merge(const SearchArgs& a, WarpCtx& w, int64_t qi, int 
       qty += __popc(m);
     }
     __syncwarp();
-    if (qty) {
-      int p0;
-      if (merge_unsorted_batch(items, num, cap, w.sk, w.sv, qty, w.nb_d, w.nb_id, &p0)) {
-        if (p0 < curr) curr = p0;
-      } else {
-        sort_like_std(w.sk, w.sv, qty, w.nb_d, w.nb_id);
-        for (int i = 0; i < qty; ++i) {
-          const int ins = sorted_insert(items, num, cap, w.sk[i], w.sv[i]);
-          if (ins < curr) curr = ins;
-        }
-      }
-    }
+    if (qty) curr = min(curr, insert_batch<kInt>(items, num, cap, w.sk, w.sv, qty, w.nb_d, w.nb_id, w.st_greedy));
     // advance to the first unused item
     while (curr < num) {
       const int t = curr + lane;
@@ -899,7 +890,7 @@ __device__ void run_query(const SearchArgs& a, char* wsmem, int slot, int64_t qi
   if (a.stats && lane == 0 && a.split != 1) {
     a.stats[qi * 4 + 0] = w.st_dist;
     a.stats[qi * 4 + 1] = w.st_expand;
-    a.stats[qi * 4 + 2] = w.st_greedy;
+    a.stats[qi * 4 + 2] = plain_count(w.st_greedy);
     a.stats[qi * 4 + 3] = w.st_bytes;
   }
   __syncwarp();
@@ -971,7 +962,7 @@ struct MultiCtx {  // lane-uniform state of one context (shared memory; lane 0 w
   int mode;        // kIdle, kEntry, kGreedy, kBeam
   int k, ef;
   int level, cur;  // greedy descent
-  float curdist;
+  float curdist;   // where the beam starts; NaN once the beam has held a NaN key
   int curr, num;   // level-0 beam (SortArrBI state)
   float top_key;   // the expansion's topKey and size (hnsw_distfunc_opt.cc:216-222)
   int size_now;
@@ -1398,16 +1389,9 @@ __global__ void __launch_bounds__(128, 8) search_multi_kernel(SearchArgs a) {
         int num = st.num, curr = st.curr;
         const int cap = max(ef, k);
         if (qty) {
-          int p0;
-          if (merge_unsorted_batch(V(c).items, num, cap, V(c).sk, V(c).sv, qty, V(c).nb_d, V(c).nb_id, &p0)) {
-            if (p0 < curr) curr = p0;
-          } else {
-            sort_like_std(V(c).sk, V(c).sv, qty, V(c).nb_d, V(c).nb_id);
-            for (int i = 0; i < qty; ++i) {
-              const int ins = sorted_insert(V(c).items, num, cap, V(c).sk[i], V(c).sv[i]);
-              if (ins < curr) curr = ins;
-            }
-          }
+          int nan = st.curdist == st.curdist ? 0 : -1;
+          curr = min(curr, insert_batch(V(c).items, num, cap, V(c).sk, V(c).sv, qty, V(c).nb_d, V(c).nb_id, nan));
+          if (nan < 0 && lane == 0) st.curdist = __int_as_float(0x7fffffff);
         }
         // advance to the first unused item
         while (curr < num) {
