@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -300,20 +301,35 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
   return NMSG_OK;
 }
 
-// Where the team kernel (one block per query, lists evaluated ahead) takes over from one warp per
-// query. Kernel time on B200, team against one-warp kernel, us:
-//   l2 1M x 128, efSearch 64:           1,200 queries 825 / 1,016   2,400: 1,012 / 1,043   4,000: 1,546 / 1,085
-//   l2sqr_sift 500K, efSearch 100:      1,000 queries 787 / 941     2,400: 1,188 / 944
-//   cosine 1M x 100, efSearch 200:      1,200 queries 1,353 / 2,355  2,400: 1,843 / 2,468 (4,000: 2,132 alone)
-//   L1 200K x 100, efSearch 100:        1,200 queries 1,018 / 2,262  4,700: 2,156 / 2,430  10,000: 3,132 / 3,017
-//   negdot 200K x 960 with SearchOld queries: 300 queries 2,650 / 6,842   4,000: 8,463 / 15,869
-// so up to 8 queries per SM for bytes, 16 for float rows, 32 for L1 / LInf (whose one-warp kernel holds
-// one row per 8 lanes), and always where SearchOld runs (one lane works its heaps in the other kernels).
+// Batches of up to this many queries run on the team kernel (one block per query, lists evaluated
+// ahead), larger ones on one warp per query; SearchOld always (one lane works its heaps in the other
+// kernels). The team's lead is the chain of memory accesses that it shortens, so it lasts to more
+// queries per SM where an expansion reads more (row length x list length), where the beam is longer and
+// where the rows lie outside L2. Time of the call on device buffers, one warp / team, us, on B200:
+//   l2 1M x 128, M 16:     efSearch 32: 592 queries 483 / 349   1,184: 515 / 545     2,368: 569 / 724
+//                          efSearch 100:                        1,184: 1,303 / 1,084  2,368: 1,444 / 1,531
+//   l2 10K x 128, M 16:    efSearch 100: 1,000 queries 432 / 363  1,600: 470 / 506   2,368: 457 / 579
+//   cosine 1M x 100, M 24: efSearch 200: 1,184 queries 1,853 / 1,242                 2,368: 1,936 / 1,990
+//   L1 200K x 100, M 16:   efSearch 100: 2,368 queries 2,337 / 1,352                 4,736: 2,458 / 2,037
+//   bytes 500K, M 16:      efSearch 50: 600 queries 553 / 431   1,184: 624 / 590
+// Fitted to both sides' times at efSearch 16 to 400 on 21 indices of the lean kernel's shapes, 3 of
+// bytes and 4 of L1 / LInf (5,000 to 1M rows, M 8 to 32): the slower side is taken at a cost of 4 to 5 %
+// (root mean square over the points) where fixed limits of 16, 8 and 32 queries per SM cost 22, 8 and
+// 18 %. Against the general kernels (other rows of L2, cosine and dot) the team leads up to 16 in nearly
+// all points.
 static int64_t team_limit(const DevIndex& d, const LaunchPlan& plan, int num_sms) {
   if (plan.with_old) return INT64_MAX;
-  if (d.dist_type == kL1 || d.dist_type == kLInf) return 32 * num_sms;
-  if (d.dist_type == kSiftL2) return 8 * num_sms;
-  return 16 * num_sms;
+  const double list = std::sqrt(std::sqrt((double)d.maxM0 * d.dim / 2048));
+  const double beam = std::sqrt(std::min(plan.region, 100) / 128.0);
+  const double far = std::min(1.0, std::pow((double)d.n * d.dim / 16e6, 0.125));
+  double per_sm = 16;
+  if (d.dist_type == kL1 || d.dist_type == kLInf)
+    per_sm = 28.5 * far;
+  else if (d.dist_type == kSiftL2)
+    per_sm = std::min(8.0, 11 * list * beam * far);
+  else if (plan.lean)
+    per_sm = std::min(16.0, 13.75 * list * beam * far);
+  return (int64_t)(per_sm * num_sms);
 }
 
 TeamParams plan_team(const DevIndex& d, const nmsg_launch_config& cfg, const LaunchPlan& plan, int64_t nq,
