@@ -823,6 +823,7 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
     if (mine) {
       d = sk[u];
       id = v.sv()[u];
+      hard = st.nan != 0;
       int lo = 0, hi = num;
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -840,13 +841,12 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
       if (old && equal > 1)  // in the order they were kept
         for (int w = 0; w < u; ++w) rank += sk[w] == d;
       if (old) {
-        hard = equal == 0;  // NaN
+        hard |= equal == 0;  // NaN
       } else {
         const bool twin = lo < num && key_of(items[lo]) == d;
-        hard = equal != 1;  // itself; 0: NaN
+        hard |= equal != 1;  // itself; 0: NaN
         hard |= twin && (lo + 1 >= num || lo + rank + 1 >= cap || key_of(items[lo + 1 < num ? lo + 1 : lo]) == d);
       }
-      hard |= st.nan != 0;
       pos = lo + rank;
       atomicMin(&st.first, lo);
       if (old && pos == cap - 1) st.edge_in = d;
