@@ -197,8 +197,10 @@ typedef struct nmsg_launch_config {
   int32_t host_copy;         /* calls on host buffers (no NMSG_DEVICE_PTRS): 0 = automatic (pageable
                                 buffers of 512 KB and more go through page-locked staging that
                                 several host threads fill and empty, with full-rate DMAs in between;
-                                page-locked buffers are copied directly), 1 = copy the caller's
-                                buffers directly */
+                                page-locked buffers of that size are copied directly; a call's smaller
+                                arrays, and pageable ones up to 1 MB, cross in one page-locked block
+                                each way, one copy for all of them), 1 = copy the caller's buffers
+                                directly */
 } nmsg_launch_config;
 
 /* Set (cfg != NULL) or reset to automatic (cfg == NULL) the launch shape used by later

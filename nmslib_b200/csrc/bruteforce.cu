@@ -1384,8 +1384,10 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
   int32_t* o_ids = dev_ptrs ? ids : reinterpret_cast<int32_t*>(s->result.as<char>() + r_ids);
   float* o_d = dev_ptrs ? dists : reinterpret_cast<float*>(s->result.as<char>() + r_dists);
   int32_t* o_c = dev_ptrs ? counts : reinterpret_cast<int32_t*>(s->result.as<char>() + r_counts);
-  // host results through the page-locked block unless direct copies are asked for or it cannot be had
-  bool pinned = !dev_ptrs && h->cfg.host_copy == 0;
+  // host results through the page-locked block unless direct copies are asked for, the caller's arrays
+  // are large and page-locked themselves, or it cannot be had
+  bool pinned = !dev_ptrs && h->cfg.host_copy == 0 &&
+                !(r_bytes >= kStageMinBytes && host_range_page_locked(ids, obytes));
   if (pinned && h->pin_out.ensure(r_bytes) != cudaSuccess) {
     cudaGetLastError();
     pinned = false;

@@ -562,10 +562,12 @@ struct CallBlock {
 };
 constexpr size_t kCallBlockBytes = 1 << 20;
 
+// Page-locked arrays of a size that staging would take (kStageMinBytes) are copied directly, in or out.
 int plan_block(nmsg_index* h, CallBlock* b, int64_t nq, size_t row_bytes, int32_t kmax, bool k_per_q, bool ef_per_q,
-               bool stats) {
-  const size_t n = (size_t)nq;
-  if (n * (8 * (size_t)kmax + 36) >= kCallBlockBytes) return NMSG_OK;
+               const void* queries, const int32_t* ids, bool stats) {
+  const size_t n = (size_t)nq, out = n * (8 * (size_t)kmax + 36), in = n * (row_bytes + 12);
+  if (out >= kCallBlockBytes) return NMSG_OK;
+  if (out >= kStageMinBytes && host_range_page_locked(ids, n * kmax * 4)) return NMSG_OK;
   size_t at = 0;
   auto take = [&](size_t bytes) {
     const size_t off = at;
@@ -573,7 +575,7 @@ int plan_block(nmsg_index* h, CallBlock* b, int64_t nq, size_t row_bytes, int32_
     return off;
   };
   CallBlock s;
-  s.in = n * (row_bytes + 12) < kCallBlockBytes;
+  s.in = in < kCallBlockBytes && !(in >= kStageMinBytes && host_range_page_locked(queries, n * row_bytes));
   if (s.in) {
     take(n * row_bytes);
     if (k_per_q) s.kq = take(n * 4);
@@ -723,6 +725,9 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   QueryParts parts;
   bool use_parts = false;
 
+  if (split)  // node, distance, 3 counts, order; range. Before the uploads: a call that fails leaves none behind
+    NMSG_CUDA(h->entry.ensure(((size_t)nq * 6 + 4) * 4, false), "cudaMalloc(level-0 entries)");
+
   // A host call of up to a megabyte of results has them in one block with the status word, which one
   // copy takes back through page-locked memory; with up to a megabyte of inputs these lie before it,
   // behind them a zeroed counter and status, and one copy brings them all. Array by array that was two
@@ -730,7 +735,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   CallBlock block;
   if (!dev_ptrs && h->cfg.host_copy == 0) {
     rc = plan_block(h, &block, nq, (size_t)dim * (u8 ? 1 : 4), kmax, k_per_q != nullptr, ef_per_q != nullptr,
-                    stats != nullptr);
+                    queries_v, ids, stats != nullptr);
     if (rc != NMSG_OK) return rc;
   }
   // inputs / outputs
@@ -841,8 +846,6 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   }
   a.nbpad = plan.nbpad;
   if (split) {
-    const size_t words = (size_t)nq * 6 + 4;  // node, distance, 3 counts, order; range
-    NMSG_CUDA(h->entry.ensure(words * 4, false), "cudaMalloc(level-0 entries)");
     int32_t* e = h->entry.as<int32_t>();
     a.entry_node = e;
     a.entry_dist = reinterpret_cast<float*>(e + nq);
