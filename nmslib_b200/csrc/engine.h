@@ -213,12 +213,12 @@ NMSG_HD inline int lean_warp_smem_bytes(int dim, int region_items, int nbpad, in
 }
 int lean_occupancy(const DevIndex& ix, int warps_per_block, int smem_per_block, int* blocks_per_sm);
 int lean_smem_bytes(const DevIndex& ix, int region_items, int nbpad, int stage_rows);
-// The team kernel for an index (team_l2.cu, team_dot.cu, team_lp.cu, team_sift.cu), 4 or 8 warps per
-// block, with or without SearchOld.
+// The team kernel for an index (team_l2.cu, team_dot.cu, team_lp.cu, team_sift.cu): 8 warps per block, or
+// 4 without SearchOld over float rows.
 void* team_kernel_l2(const DevIndex& ix, int warps, bool with_old);
 void* team_kernel_dot(const DevIndex& ix, int warps, bool with_old);
 void* team_kernel_lp(const DevIndex& ix, int warps, bool with_old);
-void* team_kernel_sift(int warps, bool with_old);
+void* team_kernel_sift(bool with_old);
 int team_occupancy(const DevIndex& ix, const TeamParams& t, bool with_old, int smem_per_block, int* blocks_per_sm);
 // Bytes one bulk row copy moves: the row rounded up to 16 bytes (the padding is zeros).
 NMSG_HD inline int bulk_row_bytes(const DevIndex& ix) { return ((ix.dim * 4 + 15) / 16) * 16; }

@@ -1999,7 +1999,7 @@ Kern team_kernel_for(const DevIndex& ix, int warps, bool with_old) {
     case kNegDot: k = team_kernel_dot(ix, warps, with_old); break;
     case kL1:
     case kLInf: k = team_kernel_lp(ix, warps, with_old); break;
-    case kSiftL2: k = team_kernel_sift(warps, with_old); break;
+    case kSiftL2: k = team_kernel_sift(with_old); break;
   }
   return reinterpret_cast<Kern>(k);
 }

@@ -5,8 +5,7 @@ namespace nmsg {
 namespace {
 template <int D>
 void* select(const DevIndex& ix, int warps, bool with_old) {
-  if (with_old)
-    return warps == 4 ? (void*)search_team_kernel<D, 0, 4, true> : (void*)search_team_kernel<D, 0, 8, true>;
+  if (with_old) return (void*)search_team_kernel<D, 0, 8, true>;
   switch (ix.n16 >> 5) {
     case 3:
       return warps == 4 ? (void*)search_team_kernel<D, 3, 4, false> : (void*)search_team_kernel<D, 3, 8, false>;

@@ -3,8 +3,7 @@
 
 namespace nmsg {
 void* team_kernel_l2(const DevIndex& ix, int warps, bool with_old) {
-  if (with_old)
-    return warps == 4 ? (void*)search_team_kernel<kTeamL2, 0, 4, true> : (void*)search_team_kernel<kTeamL2, 0, 8, true>;
+  if (with_old) return (void*)search_team_kernel<kTeamL2, 0, 8, true>;
   switch (ix.n16 >> 5) {
     case 3:
       return warps == 4 ? (void*)search_team_kernel<kTeamL2, 3, 4, false>

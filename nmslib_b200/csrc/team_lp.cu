@@ -5,8 +5,7 @@ namespace nmsg {
 namespace {
 template <int D>
 void* select(int warps, bool with_old) {
-  if (with_old)
-    return warps == 4 ? (void*)search_team_kernel<D, 0, 4, true> : (void*)search_team_kernel<D, 0, 8, true>;
+  if (with_old) return (void*)search_team_kernel<D, 0, 8, true>;
   return warps == 4 ? (void*)search_team_kernel<D, 0, 4, false> : (void*)search_team_kernel<D, 0, 8, false>;
 }
 }  // namespace

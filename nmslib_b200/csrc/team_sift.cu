@@ -2,11 +2,9 @@
 #include "team_kernel.cuh"
 
 namespace nmsg {
-void* team_kernel_sift(int warps, bool with_old) {
-  if (with_old)
-    return warps == 4 ? (void*)search_team_kernel<kTeamSift, 0, 4, true>
-                      : (void*)search_team_kernel<kTeamSift, 0, 8, true>;
-  return warps == 4 ? (void*)search_team_kernel<kTeamSift, 0, 4, false>
-                    : (void*)search_team_kernel<kTeamSift, 0, 8, false>;
+// Eight warps only: their limit ends where four would start.
+void* team_kernel_sift(bool with_old) {
+  return with_old ? (void*)search_team_kernel<kTeamSift, 0, 8, true>
+                  : (void*)search_team_kernel<kTeamSift, 0, 8, false>;
 }
 }  // namespace nmsg
