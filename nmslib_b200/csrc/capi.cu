@@ -263,15 +263,29 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
     const int nbpad = std::max(32, ((std::max(d.maxM, d.maxM0) + 31) / 32) * 32);
     const bool bulk = cfg.row_copy != 1;
     int rows = p.stage_rows;
-    // An expansion brings 9-14 new rows: 12 a round take most in one, where 8 take two row latencies
-    // (10K queries, search kernels, rows per round 4 / 8 / 12: 1M x 128, efSearch 100: 2,236 / 2,045 /
-    // 1,985 us) until the beam array or lists of more than 32 ids take the blocks' room (efSearch 128:
-    // 2,466 / 2,250 / 2,287, 320: 4,532 / 4,452 / 4,727; 1M x 100 with lists of 48, efSearch 32: 1,206 /
-    // 1,088 / 1,073, 100: 2,253 / 2,039 / 2,171, 200: 3,335 / 3,086 / 3,373, 256: 3,872 / 4,113 / 3,981).
+    // An expansion brings 9-14 new rows: 12 a round take most in one, where 8 take two row latencies and 4
+    // three or four. More rows a round cost shared memory, in two ways (10K queries, M 16 unless said, us):
+    //  * past some beam 12 rows lose resident blocks (1M x 128, rows per round 4 / 8 / 12: efSearch 100:
+    //    2,152 / 1,993 / 1,952, 256: 3,958 / 3,887 / 4,064, 400: 5,291 / 5,283 / 6,224; 1M x 100, M 24,
+    //    100: 2,244 / 2,047 / 2,168), sooner where the index lies in L2 and a row latency is short
+    //    (200K x 128: 64: 1,354 / 1,234 / 1,236, 100: 1,834 / 1,673 / 1,715; M 8: 1,928 / 1,812 / 1,707);
+    //  * eight blocks of more than 196 KB in all leave L1 28 KB in place of 60, which lists of more than
+    //    24 ids feel (200K x 128: 160: 2,454 / 2,315, 200: 2,847 / 2,914, 400: 4,572 / 4,784; 500K x 96:
+    //    256: 3,390 / 3,258, 320: 3,936 / 4,102; 300K x 128, M 24: 200: 3,287 / 3,518; but M 12:
+    //    256: 3,418 / 3,269), wide rows of short lists only while the index is not far past L2 (1M x 128:
+    //    320: 4,745 / 4,567).
     // Rows over 512 bytes keep 8 up to efSearch 160, then 4 (205 floats, efSearch 200: 4,416 / 4,761).
     if (cfg.stage_rows == 0 && d.dim <= 128) {
-      const bool short_lists = std::max(d.maxM, d.maxM0) <= 32;
-      rows = p.region <= (short_lists ? 112 : 64) ? 12 : p.region <= (short_lists ? 400 : 220) ? 8 : 4;
+      const int lists = std::max(d.maxM, d.maxM0), row_bytes = ((d.dim + 3) & ~3) * 4;
+      const double index_mb = (double)d.n * row_bytes / 1e6;
+      const bool short_lists = lists <= 32;
+      int max12 = short_lists ? 112 : 64, max8 = short_lists ? 400 : 220;
+      if (lists > 24) {
+        if (index_mb <= 126 && (short_lists ? d.dim >= 120 : d.dim > 64)) max12 = 48;
+        const int l1_kept = (196 * 1024 / 8 - 1024) / 4 - nbpad * 16 - 16 - 8 * row_bytes;  // left for the beam
+        if (!(short_lists && d.dim > 96 && index_mb >= 350)) max8 = std::min(max8, l1_kept / 8);
+      }
+      rows = p.region <= max12 ? 12 : p.region <= max8 ? 8 : 4;
     }
     if (bulk) cap_bulk_round(d, &rows);
     const int ws = lean_smem_bytes(d, p.region, nbpad, rows);
