@@ -69,9 +69,12 @@ int upload_index(nmsg_index* h) {
   std::vector<int32_t> l0((size_t)n * d.l0_pitch, 0);
   std::vector<int32_t> ext(n);
   std::vector<uint32_t> seen_in(n, 0);  // 1 + the last node whose list held each id
-  bool unique = true;
+  bool unique = true, integral = true;
+  const int64_t sample = std::max<int64_t>(1, n / 1024);
   for (int64_t i = 0; i < n; ++i) {
     const float* src = hi.vec(i);
+    if (i % sample == 0)
+      for (int e = 0; e < hi.dim && integral; ++e) integral = src[e] == std::nearbyint(src[e]);
     float* dst = vec.data() + i * d.pitch;
     for (int e = 0; e < hi.dim; ++e) dst[permuted_pos(e, hi.dim)] = src[e];
     const int32_t* lst = hi.l0(i);
@@ -83,6 +86,7 @@ int upload_index(nmsg_index* h) {
     ext[i] = hi.ext_id(i);
   }
   d.l0_unique = unique ? 1 : 0;
+  d.integral = integral ? 1 : 0;
   std::vector<int32_t> links = hi.up_links;
   if (links.empty()) links.push_back(0);
   NMSG_CUDA(h->vecs.ensure(vec.size() * 4, false), "cudaMalloc(vectors)");
@@ -151,6 +155,7 @@ int upload_sift(nmsg_index* h) {
     NMSG_CUDA(cudaMemcpy(h->norms.p, hi.sift_norms.data(), n * 4, cudaMemcpyHostToDevice), "upload norms");
     d.norms = h->norms.as<int32_t>();
   }
+  d.integral = 1;
   d.vecs_u8 = h->vecs.as<uint8_t>();
   d.l0 = h->l0.as<int32_t>();
   d.up_off = h->up_off.as<int64_t>();
@@ -316,10 +321,9 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
 }
 
 // Batches of up to this many queries run on the team kernel (one block per query, lists evaluated
-// ahead), larger ones on one warp per query; SearchOld always (one lane works its heaps in the other
-// kernels). The team's lead is the chain of memory accesses that it shortens, so it lasts to more
-// queries per SM where an expansion reads more (row length x list length), where the beam is longer and
-// where the rows lie outside L2. Time of the call on device buffers, one warp / team, us, on B200:
+// ahead), larger ones on one warp per query. The team's lead is the chain of memory accesses that it
+// shortens, so it lasts to more queries per SM where an expansion reads more (row length x list length),
+// where the beam is longer and where the rows lie outside L2. Time of the call on device buffers, one warp / team, us, on B200:
 //   l2 1M x 128, M 16:     efSearch 32: 592 queries 483 / 349   1,184: 515 / 545     2,368: 569 / 724
 //                          efSearch 100:                        1,184: 1,303 / 1,084  2,368: 1,444 / 1,531
 //   l2 10K x 128, M 16:    efSearch 100: 1,000 queries 432 / 363  1,600: 470 / 506   2,368: 457 / 579
@@ -331,13 +335,23 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
 // (root mean square over the points) where fixed limits of 16, 8 and 32 queries per SM cost 22, 8 and
 // 18 %. Against the general kernels (other rows of L2, cosine and dot) the team leads up to 16 in nearly
 // all points.
+// SearchOld: one lane works the heaps of the one-warp kernel, which the team's walk does without, so its
+// lead lasts four to five times longer; but where distances are often equal (rows of whole numbers) the
+// walk tends to end in a second search with heaps. The calls on host arrays, one warp / team, us:
+//   cosine 200K x 100, M 16: efSearch 100: 1,000 queries 2,389 / 887  10,000: 5,133 / 4,653
+//                            efSearch 20:                             10,000: 1,783 / 2,521
+//   l2 1M x 128, M 16 (whole numbers): efSearch 100: 1,000 queries 3,194 / 3,079  4,000: 3,910 / 4,359
+//   negdot 1M x 960: 8,000 queries, efSearch 64 to 1,024, 182 of them SearchOld: 40,400 / 23,500
+// Fitted to 15 indices, efSearch 20 to 1,000, 1 to 54 queries per SM: 6 % (root mean square) against 20 %
+// (whole numbers) and 12 % for the team always.
 static int64_t team_limit(const DevIndex& d, const LaunchPlan& plan, int num_sms) {
-  if (plan.with_old) return INT64_MAX;
   const double list = std::sqrt(std::sqrt((double)d.maxM0 * d.dim / 2048));
   const double beam = std::sqrt(std::min(plan.region, 100) / 128.0);
   const double far = std::min(1.0, std::pow((double)d.n * d.dim / 16e6, 0.125));
   double per_sm = 16;
-  if (d.dist_type == kL1 || d.dist_type == kLInf)
+  if (plan.with_old)
+    per_sm = d.integral ? 16 * list : 64 * list * beam * far;
+  else if (d.dist_type == kL1 || d.dist_type == kLInf)
     per_sm = 28.5 * far;
   else if (d.dist_type == kSiftL2)
     per_sm = std::min(8.0, 11 * list * beam * far);

@@ -102,6 +102,8 @@ struct DevIndex {
   int row_bytes = 0;                // algorithmic bytes of one row: 4 dim, or 132 for l2sqr_sift
   int l0_unique = 0;                // 1: no level-0 list repeats an id (checked at upload), so a
                                     // list's visited checks need no duplicate vote
+  int integral = 0;                 // 1: the rows hold whole numbers (sampled at upload), whose
+                                    // distances are often equal
 };
 
 // Position of element e of a vector in the permuted device row.
