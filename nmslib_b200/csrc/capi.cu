@@ -341,16 +341,17 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
 //   cosine 200K x 100, M 16: efSearch 100: 1,000 queries 2,389 / 887  10,000: 5,133 / 4,653
 //                            efSearch 20:                             10,000: 1,783 / 2,521
 //   l2 1M x 128, M 16 (whole numbers): efSearch 100: 1,000 queries 3,194 / 3,079  4,000: 3,910 / 4,359
+//     efSearch 64 to 1,024, one in 40 SearchOld: 4,500 queries ahead by 5 %        10,000: behind by 14 %
 //   negdot 1M x 960: 8,000 queries, efSearch 64 to 1,024, 182 of them SearchOld: 40,400 / 23,500
-// Fitted to 15 indices, efSearch 20 to 1,000, 1 to 54 queries per SM: 6 % (root mean square) against 20 %
-// (whole numbers) and 12 % for the team always.
+// Fitted to 15 indices, efSearch 20 to 1,000, 1 to 54 queries per SM: 6 to 7 % (root mean square) against
+// 20 (whole numbers) and 12 % for the team always; mixed batches on 11 indices, 300 to 10,000 queries: 3 %.
 static int64_t team_limit(const DevIndex& d, const LaunchPlan& plan, int num_sms) {
   const double list = std::sqrt(std::sqrt((double)d.maxM0 * d.dim / 2048));
   const double beam = std::sqrt(std::min(plan.region, 100) / 128.0);
   const double far = std::min(1.0, std::pow((double)d.n * d.dim / 16e6, 0.125));
   double per_sm = 16;
   if (plan.with_old)
-    per_sm = d.integral ? 16 * list : 64 * list * beam * far;
+    per_sm = d.integral ? (36 - 20 * plan.old_share) * list : 64 * list * beam;
   else if (d.dist_type == kL1 || d.dist_type == kLInf)
     per_sm = 28.5 * far;
   else if (d.dist_type == kSiftL2)
@@ -646,6 +647,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   // per-query parameters and capacity of the shared-memory region
   int region = 1;
   bool any_old = false;
+  int64_t num_old = 0;
   for (int64_t i = 0; i < nq; ++i) {
     const int kq = k_per_q ? k_per_q[i] : k;
     const int eq = ef_per_q ? ef_per_q[i] : ef;
@@ -654,6 +656,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
     if (eq < 0) return fail(NMSG_ERR_BAD_ARG, "ef must be non-negative");
     const bool old = algo == NMSG_ALGO_OLD || (algo == NMSG_ALGO_HYBRID && eq >= 1000);
     any_old |= old;
+    num_old += old;
     // V1Merge keeps its sorted array of max(ef, k) items; SearchOld its closest-set heap (ef + 1)
     // and the k results
     region = std::max(region, old ? eq + 1 + kq : std::max(eq, kq));
@@ -698,6 +701,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   int rc = plan_launch(d, h->cfg, region, any_old, plain, &plan, &perr);
   if (rc != NMSG_OK) return fail(rc, perr);
   region = plan.region;
+  plan.old_share = !any_old ? 0.0 : k_per_q || ef_per_q ? (double)num_old / (double)nq : 1.0;
   a.region_items = plan.region;
   a.hash_log2 = plan.hash_log2;
   a.stage_rows = plan.stage_rows;

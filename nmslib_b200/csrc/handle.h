@@ -39,6 +39,7 @@ struct LaunchPlan {
   int wpb = kWarpsPerBlock;
   int blocks_per_sm = 0;
   bool with_old = false;
+  double old_share = 0;   // share of the batch's queries that take SearchOld (the caller's to set)
   int ctx = 1;            // queries per persistent warp (> 1: search_multi_kernel)
   bool bulk_rows = false; // search_multi_kernel stages rows with bulk copies
   bool lean = false;      // search_lean_kernel
