@@ -642,6 +642,11 @@ __device__ DF exact_key_lane(const float* __restrict__ q, const float* __restric
   return DF{hi, __double2float_rn(acc - (double)hi)};
 }
 
+__device__ __forceinline__ uint32_t desc_key(float f) {  // larger float, larger key
+  const uint32_t b = __float_as_uint(f);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
 // One block per query:
 //  1. B_k = the k-th largest BF16 key among the candidates (a radix selection, 8 bits a pass);
 //  2. only candidates with BF16 key >= B_k - 2 eps can be in the exact top k (the k candidates
@@ -652,27 +657,21 @@ __device__ DF exact_key_lane(const float* __restrict__ q, const float* __restric
 //  4. tau = exact k-th key - eps (rounded down, less one ulp of the double-float's high part):
 //     the candidates are real base vectors, so their exact k-th key is at most the true k-th
 //     key, and every true top-k vector has a BF16 key >= tau.
-// The candidates of up to kRerankCap rows are gathered from their lists into shared memory once; more
+// The candidates of up to CAP rows are gathered from their lists into shared memory once; more
 // of them are read from the lists at each pass. With one warp per query (k passes over the lists for
 // B_k, then k rounds of warp maxima per 32 candidates) small batches waited on that one warp: 333
 // queries, k 32, 1M x 100 cosine took 886 us (sample) and 1,430 us (final) in this kernel, against
 // 48 and 130 us in the scans that feed it; with a block per query 22 and 164 us. 10,000 queries, k 10,
-// 1M x 128 l2: 206 and 398 us -> 176 and 231. Latency-bound: the list counts, four histogram passes,
+// 1M x 128 l2: 205 and 410 us -> 69 and 92. Latency-bound: the list counts, four histogram passes,
 // one row read per candidate and a rank loop, each behind a barrier.
-constexpr int kRerankThreads = 256;
-constexpr int kRerankCap = 2048;  // candidates held in shared memory
-constexpr int kRerankBuf = 512;   // rows with exact keys at once, besides the k best so far
-
-__device__ __forceinline__ uint32_t desc_key(float f) {  // larger float, larger key
-  const uint32_t b = __float_as_uint(f);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-__global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
-  __shared__ int32_t c_id[kRerankCap];
-  __shared__ float c_key[kRerankCap];
-  __shared__ int32_t b_id[kRerankBuf + CAND];
-  __shared__ DF b_key[kRerankBuf + CAND];
+// T threads per block, CAP candidates held in shared memory, BUF rows with exact keys at once besides
+// the k best so far.
+template <int T, int CAP, int BUF>
+__global__ void __launch_bounds__(T) rerank_kernel(RerankArgs a) {
+  __shared__ int32_t c_id[CAP];
+  __shared__ float c_key[CAP];
+  __shared__ int32_t b_id[BUF + CAND];
+  __shared__ DF b_key[BUF + CAND];
   __shared__ int hist[256];
   __shared__ int s_total, s_found, s_over, s_fill, s_want, s_have;
   __shared__ uint32_t s_prefix;
@@ -690,7 +689,7 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
   __syncthreads();
   {
     int total = 0, found = 0, over = 0;
-    for (int l = tid; l < a.n_lists; l += kRerankThreads) {
+    for (int l = tid; l < a.n_lists; l += T) {
       const int cnt = lc[l];
       found += cnt;
       total += min(cnt, a.list_len);
@@ -702,12 +701,12 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
   }
   __syncthreads();
   const int total = s_total;
-  const bool held = total <= kRerankCap;
+  const bool held = total <= CAP;
   // few long lists: 8 threads each; many short ones: a thread each
-  const int per = a.n_lists <= kRerankThreads ? 8 : 1;
+  const int per = a.n_lists <= T ? 8 : 1;
   const int sub = tid % per;
   if (held) {
-    for (int l = tid / per; l < a.n_lists; l += kRerankThreads / per) {
+    for (int l = tid / per; l < a.n_lists; l += T / per) {
       const int cnt = min(lc[l], a.list_len);
       if (cnt == 0) continue;
       int at = 0;
@@ -729,7 +728,7 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
       s_want = a.k;
     }
     for (int shift = 24; shift >= 0; shift -= 8) {
-      hist[tid] = 0;
+      for (int b = tid; b < 256; b += T) hist[b] = 0;
       __syncthreads();
       const uint32_t prefix = s_prefix;
       auto count = [&](float v) {
@@ -737,9 +736,9 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
         if (shift == 24 || (d >> (shift + 8)) == prefix) atomicAdd(&hist[(d >> shift) & 255], 1);
       };
       if (held) {
-        for (int t = tid; t < total; t += kRerankThreads) count(c_key[t]);
+        for (int t = tid; t < total; t += T) count(c_key[t]);
       } else {
-        for (int l = tid / per; l < a.n_lists; l += kRerankThreads / per) {
+        for (int l = tid / per; l < a.n_lists; l += T / per) {
           const int cnt = min(lc[l], a.list_len);
           for (int e = sub; e < cnt; e += per) count(keys[(size_t)l * a.list_len + e]);
         }
@@ -777,19 +776,19 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
   __syncthreads();
   auto cut_back = [&]() {  // exact keys of the new rows, then the k best of all to the front
     const int have = s_have, fill = s_fill;
-    for (int t = have + tid; t < fill; t += kRerankThreads) {
+    for (int t = have + tid; t < fill; t += T) {
       const int id = b_id[t];
       DF xn{0.0f, 0.0f};
       if (a.l2) xn = DF{a.xn_hi[id], a.xn_lo[id]};
       b_key[t] = exact_key_lane(qv, a.x + (size_t)id * a.dim, a.dim, a.l2, xn);
     }
     __syncthreads();
-    constexpr int kMine = (kRerankBuf + CAND + kRerankThreads - 1) / kRerankThreads;
+    constexpr int kMine = (BUF + CAND + T - 1) / T;
     int rank[kMine], id[kMine];
     DF key[kMine];
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
-      const int t = tid + i * kRerankThreads;
+      const int t = tid + i * T;
       rank[i] = 0x7fffffff;
       if (t >= fill) continue;
       key[i] = b_key[t];
@@ -817,17 +816,17 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
     if (in && key >= cut) b_id[atomicAdd(&s_fill, 1)] = id;
   };
   if (held) {
-    for (int t0 = 0; t0 < total; t0 += kRerankThreads) {
+    for (int t0 = 0; t0 < total; t0 += T) {
       const int t = t0 + tid;
       offer(t < total, t < total ? c_key[t] : 0.0f, t < total ? c_id[t] : 0);
       __syncthreads();
-      const bool full = s_fill > kRerankBuf + CAND - kRerankThreads;
+      const bool full = s_fill > BUF + CAND - T;
       __syncthreads();  // read by all before the next step adds to it
       if (full) cut_back();
     }
   } else {
     // one entry of every thread's list a step, so that a step adds at most a buffer's slack
-    for (int l0 = 0; l0 < a.n_lists; l0 += kRerankThreads / per) {
+    for (int l0 = 0; l0 < a.n_lists; l0 += T / per) {
       const int l = l0 + tid / per;
       const int cnt = l < a.n_lists ? min(lc[l], a.list_len) : 0;
       for (int e0 = 0; __syncthreads_or(e0 < cnt); e0 += per) {
@@ -836,7 +835,7 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
         const size_t at = (size_t)l * a.list_len + e;
         offer(in, in ? keys[at] : 0.0f, in ? ids[at] : 0);
         __syncthreads();
-        if (s_fill > kRerankBuf + CAND - kRerankThreads) cut_back();
+        if (s_fill > BUF + CAND - T) cut_back();
       }
     }
   }
@@ -858,6 +857,22 @@ __global__ void __launch_bounds__(kRerankThreads) rerank_kernel(RerankArgs a) {
       if (s_over) atomicAdd(a.summary + 1, 1);
     }
   }
+}
+
+// 256 threads a query while that leaves SMs short of work; beyond, 128, and past 16 queries per SM 64 for
+// short results: many queries are bound by the barriers of all resident blocks, of which smaller ones
+// make more. Both reranks' time, one warp per query (the form before) / 256 / 128 / 64 threads, us:
+//   300 queries, 1M x 128 l2, k 32: 1,365 / 45 / 61 / 160;   1,000, 200K x 100 cosine, k 10: 751 / 176 / 145 / 277
+//   10,000 queries: 5,000 x 128 l2, k 10: 157 / 308 / 185 / 120;   1M x 128, k 1: 136 / 360 / 219 / 131,
+//   k 32: 1,769 / 458 / 341 / 346;   50K x 300 dot, k 32: 3,112 / 1,018 / 911 / 1,061
+void launch_rerank(const RerankArgs& r, int num_sms, cudaStream_t st) {
+  const unsigned nq = (unsigned)r.nq;
+  if (r.nq <= 4 * num_sms)
+    rerank_kernel<256, 2048, 512><<<nq, 256, 0, st>>>(r);
+  else if (r.nq > 16 * num_sms && r.k <= 16)
+    rerank_kernel<64, 512, 128><<<nq, 64, 0, st>>>(r);
+  else
+    rerank_kernel<128, 1024, 256><<<nq, 128, 0, st>>>(r);
 }
 
 }  // namespace
@@ -1219,8 +1234,9 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
   const int s_tiles = std::min(n_tiles, std::max(16, n_tiles / 16));
   const int s_step = n_tiles / s_tiles;
   // (chunks of at least 4 tiles; the split with the least of: tiles the busiest CTA visits plus the
-  // rerank's cost of the candidate lists each chunk adds per query, which measured on B200 as about
-  // 14 tile visits per chunk for 10K queries, in proportion to the query count)
+  // rerank's cost of the candidate lists each chunk adds per query. 14 tile visits per chunk for 10K
+  // queries, in proportion to the query count, was measured with one warp per query in the rerank,
+  // which is faster now: an upper bound)
   int s_chunks = 1, s_chunk_tiles = s_tiles;
   {
     const double per_chunk = 14.0 * (double)nq / 10000.0;
@@ -1351,7 +1367,7 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
   ra.out_keys = s->out_key.as<DF>();
   ra.out_count = s->out_cnt.as<int32_t>();
   ra.tau = s->tau.as<float>();
-  rerank_kernel<<<(unsigned)nq, kRerankThreads, 0, st>>>(ra);
+  launch_rerank(ra, h->num_sms, st);
   BF_CUDA(cudaGetLastError(), "rerank (sample)");
 
   // 2. every base tile, collecting BF16 keys >= tau; exact rerank of the collection. A query
@@ -1400,7 +1416,7 @@ extern "C" NMSG_API int nmsg_bruteforce_knn(nmsg_index* h, const float* queries,
                                                                                                    gb);
     BF_CUDA(cudaGetLastError(), "brute-force scan");
     rb.only = attempt == 0 ? nullptr : s->qact.as<uint8_t>();  // the other queries keep their results
-    rerank_kernel<<<(unsigned)nq, kRerankThreads, 0, st>>>(rb);
+    launch_rerank(rb, h->num_sms, st);
     BF_CUDA(cudaGetLastError(), "rerank");
     // the results follow at once: an overflow, which writes them again, is rare, and waiting for the
     // summary first cost a round trip and a pageable copy per array (333 queries: 140 of 530 us)
