@@ -198,7 +198,7 @@ typedef struct nmsg_launch_config {
                                 buffers of 512 KB and more go through page-locked staging that
                                 several host threads fill and empty, with full-rate DMAs in between;
                                 page-locked buffers of that size are copied directly; a call's smaller
-                                arrays, and pageable ones up to 1 MB, cross in one page-locked block
+                                arrays, and pageable ones up to 900 KB, cross in one page-locked block
                                 each way, one copy for all of them), 1 = copy the caller's buffers
                                 directly */
 } nmsg_launch_config;

@@ -589,7 +589,9 @@ struct CallBlock {
   bool in = false;  // the inputs are part of it
   size_t kq = 0, efq = 0, order = 0, ctl = 0, ids = 0, dists = 0, counts = 0, stats = 0, bytes = 0;
 };
-constexpr size_t kCallBlockBytes = 1 << 20;
+// Past this, several host threads around staged copies are faster than one copy and one thread (10K x 128,
+// efSearch 16, k 10, results of 696 / 870 / 986 KB: 432 / 480 / 531 us in a block, 498 / 493 / 518 staged).
+constexpr size_t kCallBlockBytes = 900 * 1024;
 
 // Page-locked arrays of a size that staging would take (kStageMinBytes) are copied directly, in or out.
 int plan_block(nmsg_index* h, CallBlock* b, int64_t nq, size_t row_bytes, int32_t kmax, bool k_per_q, bool ef_per_q,
@@ -760,8 +762,8 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   if (split)  // node, distance, 3 counts, order; range. Before the uploads: a call that fails leaves none behind
     NMSG_CUDA(h->entry.ensure(((size_t)nq * 6 + 4) * 4, false), "cudaMalloc(level-0 entries)");
 
-  // A host call of up to a megabyte of results has them in one block with the status word, which one
-  // copy takes back through page-locked memory; with up to a megabyte of inputs these lie before it,
+  // A host call with results of up to kCallBlockBytes has them in one block with the status word, which one
+  // copy takes back through page-locked memory; with as few bytes of inputs these lie before it,
   // behind them a zeroed counter and status, and one copy brings them all. Array by array that was two
   // memsets and a pageable copy of about 15 us each: one query over 10K x 128 198 -> 150 us per call.
   CallBlock block;
