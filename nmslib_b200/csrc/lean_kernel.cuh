@@ -585,7 +585,10 @@ void* lean_tail(bool two) {
   return two ? (void*)search_lean_kernel<NF, HALF, SP, 2, true> : (void*)search_lean_kernel<NF, HALF, SP, 1, true>;
 }
 
-// The instantiation for this index's row length and list length (SP fixed by the file), or null.
+// The instantiation for this index's row length and list length (SP fixed by the file), or null. Each length
+// is two more kernels per distance; the others run on the general kernel, which is slower (10,000 queries of
+// l2 200K rows, M 16, efSearch 64: 32 / 80 / 112 / 160 / 224 floats there 1,331 / 1,540 / 1,633 / 1,889 /
+// 2,367 us; 33 / 81 / 113 / 256 here 992 / 1,144 / 1,303 / 1,974).
 template <int SP>
 void* lean_kernel_select(const DevIndex& ix) {
   const bool two = std::max(ix.maxM, ix.maxM0) > 32;

@@ -6,6 +6,7 @@ namespace {
 template <int D>
 void* select(const DevIndex& ix, int warps, bool with_old) {
   if (with_old) return (void*)search_team_kernel<D, 0, 8, true>;
+  // as in team_l2.cu; cosine 1M x 100, M 24, efSearch 200, 600 / 2,000 queries: 1,090 / 2,026 -> 963 / 1,734 us
   switch (ix.n16 >> 5) {
     case 3:
       return warps == 4 ? (void*)search_team_kernel<D, 3, 4, false> : (void*)search_team_kernel<D, 3, 8, false>;
