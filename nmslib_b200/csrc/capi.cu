@@ -323,7 +323,8 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
 // Batches of up to this many queries run on the team kernel (one block per query, lists evaluated
 // ahead), larger ones on one warp per query. The team's lead is the chain of memory accesses that it
 // shortens, so it lasts to more queries per SM where an expansion reads more (row length x list length),
-// where the beam is longer and where the rows lie outside L2. Time of the call on device buffers, one warp / team, us, on B200:
+// where the beam is longer and where the rows lie outside L2. Time of the call on device buffers, one
+// warp / team, us, on B200:
 //   l2 1M x 128, M 16:     efSearch 32: 592 queries 483 / 349   1,184: 515 / 545     2,368: 569 / 724
 //                          efSearch 100:                        1,184: 1,303 / 1,084  2,368: 1,444 / 1,531
 //   l2 10K x 128, M 16:    efSearch 100: 1,000 queries 432 / 363  1,600: 470 / 506   2,368: 457 / 579
@@ -389,8 +390,7 @@ TeamParams plan_team(const DevIndex& d, const nmsg_launch_config& cfg, const Lau
     if (bps >= 1 && (t.table_log2 <= least || (int64_t)bps * num_sms >= nq)) break;
   }
   if (bps < 1) return none;  // a beam that leaves no room for the table
-  t.resident = bps * num_sms;
-  t.blocks = (int)std::min<int64_t>(nq, t.resident);
+  t.blocks = (int)std::min<int64_t>(nq, (int64_t)bps * num_sms);
   return t;
 }
 
@@ -714,9 +714,11 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
                                                         : bps * h->num_sms)
                                : blocks * wpb * plan.ctx;
   if (!plain) a.team = plan_team(d, h->cfg, plan, nq, h->num_sms);
-  // visited sets: as many as any batch size can have resident at this beam size, so that batches of
-  // growing size do not grow them (an allocation in mid-service, refused under stream capture)
-  const int slots = std::max(warp_slots, a.team.resident);
+  // visited sets: as many as the one-warp kernels have resident at this beam size, whatever the batch's
+  // size, so that growing batches do not grow them (an allocation in mid-service, refused under stream
+  // capture). The team kernel rarely has more blocks; it makes do with these.
+  const int slots = warp_slots;
+  a.team.blocks = std::min(a.team.blocks, slots);
   a.ctx_per_warp = plan.ctx;
   a.bulk_rows = plan.bulk_rows ? 1 : 0;
   a.lean = plan.lean ? 1 : 0;

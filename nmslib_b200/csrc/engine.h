@@ -125,7 +125,6 @@ struct TeamLayout {  // byte offsets of a block's shared-memory pieces (its stat
 struct TeamParams {
   int warps = 0;       // warps per block; 0: the team kernel is not used
   int blocks = 0;      // grid
-  int resident = 0;    // blocks the GPU holds at once
   int table_log2 = 0;  // entries of the block's table of evaluated ids
   int spec = 0;        // candidate lists evaluated per round, at most kTeamSlots
   int lcap = 0;        // ids per evaluated list (maxM0 rounded up to 32)
