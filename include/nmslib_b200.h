@@ -124,7 +124,8 @@ NMSG_API int nmsg_set_query_params(nmsg_index* index, int ef, int algo);
  *   kmax: row stride of ids/dists (>= every k used).
  *   ids   [nq * kmax]: external ids (the ids stored in each node's object header), -1 padding.
  *   dists [nq * kmax]: distances in ascending order, +inf padding. l2 reports SQUARED
- *                      distance, as the reference's optimized path does.
+ *                      distance, as the reference's optimized path does. A distance that is not a
+ *                      number (an infinite coordinate against a zero) counts as infinite.
  *   counts[nq]: results per query, min(k, found).
  *   stats [nq * 4] (optional): distance evaluations, level-0 expansions, upper-level list
  *                      scans, algorithmic bytes read.

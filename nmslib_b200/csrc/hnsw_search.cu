@@ -237,7 +237,7 @@ __device__ void compute_dists(const DevIndex& ix, const float* __restrict__ q, c
       const bool act = idx < n;
       const float* row = ix.vecs + (int64_t)(act ? ids[idx] : 0) * ix.pitch;
       const float d = lp_group_dist<true>(ix, q, row, act);
-      if (act && j == 0) out[idx] = d;
+      if (act && j == 0) out[idx] = kept_dist(d);
     }
     __syncwarp();
   } else {
@@ -280,7 +280,7 @@ __device__ void compute_dists(const DevIndex& ix, const float* __restrict__ q, c
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const float d = combine(ix, acc[r], rows[r], q);
-        if (act[r] && j == 0) out[base + g + 4 * r] = d;
+        if (act[r] && j == 0) out[base + g + 4 * r] = kept_dist(d);
       }
     }
     __syncwarp();
@@ -346,7 +346,7 @@ __device__ void compute_dists_staged(const DevIndex& ix, const float* __restrict
         acc = fma_term(code, qv.y, x.y, acc);
       }
       const float d = combine(ix, acc, row, q);
-      if (act && j == 0) out[base + r] = d;
+      if (act && j == 0) out[base + r] = kept_dist(d);
     }
     __syncwarp();
   }
@@ -643,8 +643,6 @@ __device__ void search_v1merge(const SearchArgs& a, WarpCtx& w, int64_t qi, int 
   const int cap = max(ef, k);
   uint2* items = w.items;
   int num = 1;
-  constexpr bool kInt = R == kSiftGather;
-  if (!kInt && !(curdist == curdist)) w.st_greedy = ~w.st_greedy;  // see insert_batch
   if (lane == 0) items[0] = make_item(curdist, cur, false);
   visit_one(w, cur);
   int curr = 0;
@@ -692,7 +690,18 @@ __device__ void search_v1merge(const SearchArgs& a, WarpCtx& w, int64_t qi, int 
       qty += __popc(m);
     }
     __syncwarp();
-    if (qty) curr = min(curr, insert_batch<kInt>(items, num, cap, w.sk, w.sv, qty, w.nb_d, w.nb_id, w.st_greedy));
+    if (qty) {
+      int p0;
+      if (merge_unsorted_batch(items, num, cap, w.sk, w.sv, qty, w.nb_d, w.nb_id, &p0)) {
+        if (p0 < curr) curr = p0;
+      } else {
+        sort_like_std(w.sk, w.sv, qty, w.nb_d, w.nb_id);
+        for (int i = 0; i < qty; ++i) {
+          const int ins = sorted_insert(items, num, cap, w.sk[i], w.sv[i]);
+          if (ins < curr) curr = ins;
+        }
+      }
+    }
     // advance to the first unused item
     while (curr < num) {
       const int t = curr + lane;
@@ -890,7 +899,7 @@ __device__ void run_query(const SearchArgs& a, char* wsmem, int slot, int64_t qi
   if (a.stats && lane == 0 && a.split != 1) {
     a.stats[qi * 4 + 0] = w.st_dist;
     a.stats[qi * 4 + 1] = w.st_expand;
-    a.stats[qi * 4 + 2] = plain_count(w.st_greedy);
+    a.stats[qi * 4 + 2] = w.st_greedy;
     a.stats[qi * 4 + 3] = w.st_bytes;
   }
   __syncwarp();
@@ -962,7 +971,7 @@ struct MultiCtx {  // lane-uniform state of one context (shared memory; lane 0 w
   int mode;        // kIdle, kEntry, kGreedy, kBeam
   int k, ef;
   int level, cur;  // greedy descent
-  float curdist;   // where the beam starts; NaN once the beam has held a NaN key
+  float curdist;
   int curr, num;   // level-0 beam (SortArrBI state)
   float top_key;   // the expansion's topKey and size (hnsw_distfunc_opt.cc:216-222)
   int size_now;
@@ -1302,7 +1311,7 @@ __global__ void __launch_bounds__(128, 8) search_multi_kernel(SearchArgs a) {
             out = V(c).nb_d;
           }
         const float d = staged_row_dist(ix, q, stage + (act ? r : 0) * ix.pitch);
-        if (act && (lane & 7) == 0) out[gr - off[cc]] = d;
+        if (act && (lane & 7) == 0) out[gr - off[cc]] = kept_dist(d);
       }
       __syncwarp();
     }
@@ -1389,9 +1398,16 @@ __global__ void __launch_bounds__(128, 8) search_multi_kernel(SearchArgs a) {
         int num = st.num, curr = st.curr;
         const int cap = max(ef, k);
         if (qty) {
-          int nan = st.curdist == st.curdist ? 0 : -1;
-          curr = min(curr, insert_batch(V(c).items, num, cap, V(c).sk, V(c).sv, qty, V(c).nb_d, V(c).nb_id, nan));
-          if (nan < 0 && lane == 0) st.curdist = __int_as_float(0x7fffffff);
+          int p0;
+          if (merge_unsorted_batch(V(c).items, num, cap, V(c).sk, V(c).sv, qty, V(c).nb_d, V(c).nb_id, &p0)) {
+            if (p0 < curr) curr = p0;
+          } else {
+            sort_like_std(V(c).sk, V(c).sv, qty, V(c).nb_d, V(c).nb_id);
+            for (int i = 0; i < qty; ++i) {
+              const int ins = sorted_insert(V(c).items, num, cap, V(c).sk[i], V(c).sv[i]);
+              if (ins < curr) curr = ins;
+            }
+          }
         }
         // advance to the first unused item
         while (curr < num) {

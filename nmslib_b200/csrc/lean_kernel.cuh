@@ -224,7 +224,7 @@ __device__ bool lean_rows(const DevIndex& ix, LeanWarp& w, const LeanQuery<NF, H
       const int r = r0 + g;
       const bool act = r < rows;
       const float d = lean_row_dist<NF, HALF, SP, TAIL>(ix, q, w.stage + (act ? r : 0) * kDim);
-      if (act && (lane & 7) == 0) w.nb_d[base + r] = d;
+      if (act && (lane & 7) == 0) w.nb_d[base + r] = kept_dist(d);
     }
     __syncwarp();
   }
@@ -237,8 +237,7 @@ __device__ bool lean_rows(const DevIndex& ix, LeanWarp& w, const LeanQuery<NF, H
 // keys below it) + (kept keys below it). When no kept key equals another kept key or an array key,
 // that is the array that sorting the batch and inserting its items one by one with
 // push_or_replace_non_empty_exp (sort_arr_bi.h:159-199) leaves, truncated to cap, and the smallest
-// insertion index is the kept minimum's. With such a tie, or a kept NaN, it returns false and changes
-// nothing.
+// insertion index is the kept minimum's. With such a tie it returns false and changes nothing.
 __device__ __forceinline__ bool lean_merge64(uint2* items, int& num, int cap, float d, int idt, bool keep,
                                              int* first_pos) {
   const int lane = lane_id();
@@ -248,7 +247,7 @@ __device__ __forceinline__ bool lean_merge64(uint2* items, int& num, int cap, fl
   const uint2 it1 = h1 ? items[lane + 32] : make_uint2(0u, 0u);
   const float k0 = key_of(it0), k1 = key_of(it1);
   int rank = 0, lb = 0, c0 = 0, c1 = 0;
-  bool tie = keep && !(d == d);
+  bool tie = false;
   for (unsigned mm = km; mm; mm &= mm - 1) {
     const int u = __ffs(mm) - 1;
     const float ku = __shfl_sync(kFull, d, u);
@@ -415,7 +414,6 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
   // ---- level 0 (hnsw_distfunc_opt.cc:200-283)
   const int cap = max(ef, k);
   int num = 1, curr = 0;
-  if (!(curdist == curdist)) w.st_greedy = ~w.st_greedy;  // see insert_batch
   if (lane == 0) {
     w.items[0] = make_item(curdist, cur, false);
     w.vis[cur] = epoch;
@@ -474,7 +472,7 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
         const int idt = valid ? w.nb_id[lane] : 0;
         const bool keep = valid && ((d < top_key) || (size_now < ef));
         int p0 = 0x7fffffff;
-        merged = !__any_sync(kFull, keep) || (w.st_greedy >= 0 && lean_merge64(w.items, num, cap, d, idt, keep, &p0));
+        merged = !__any_sync(kFull, keep) || lean_merge64(w.items, num, cap, d, idt, keep, &p0);
         if (p0 < curr) curr = p0;
       }
     }
@@ -500,8 +498,18 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
       qty += __popc(mk);
     }
     __syncwarp();
-    if (qty && !merged)
-      curr = min(curr, insert_batch(w.items, num, cap, w.sk, w.sv, qty, w.nb_d, w.nb_id, w.st_greedy));
+    if (qty && !merged) {
+      int p0;
+      if (merge_unsorted_batch(w.items, num, cap, w.sk, w.sv, qty, w.nb_d, w.nb_id, &p0)) {
+        if (p0 < curr) curr = p0;
+      } else {
+        sort_like_std(w.sk, w.sv, qty, w.nb_d, w.nb_id);
+        for (int i = 0; i < qty; ++i) {
+          const int ins = sorted_insert(w.items, num, cap, w.sk[i], w.sv[i]);
+          if (ins < curr) curr = ins;
+        }
+      }
+    }
     // advance to the first unused item
     while (curr < num) {
       const int t = curr + lane;
@@ -520,7 +528,7 @@ __device__ bool lean_query(const SearchArgs& a, LeanWarp& w, int64_t qi, uint8_t
   if (a.stats && lane == 0) {
     a.stats[qi * 4 + 0] = w.st_dist;
     a.stats[qi * 4 + 1] = w.st_expand;
-    a.stats[qi * 4 + 2] = plain_count(w.st_greedy);
+    a.stats[qi * 4 + 2] = w.st_greedy;
     a.stats[qi * 4 + 3] = (int64_t)ix.row_bytes * w.st_dist + 4LL * w.st_list_ints;
   }
   __syncwarp();

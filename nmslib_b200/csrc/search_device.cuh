@@ -38,6 +38,11 @@ __device__ __forceinline__ uint32_t ordered_key(float f) {
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// A distance as the searches keep it: NaN (an infinite query coordinate against a zero, for one) counts
+// as infinite. Every key then has its place in an order, without which the merges' positions collide and
+// leave others unwritten, and the sorts run past their ends.
+__device__ __forceinline__ float kept_dist(float d) { return fminf(d, __int_as_float(0x7f800000)); }
+
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
@@ -231,14 +236,13 @@ __device__ void lib_std_sort(KV a, int n) {
 // Order sk/sv[0..n) as std::sort would. Warp-cooperative; tmpk/tmpv are scratch of length n.
 // Without equal keys every correct sort gives the same order, and for n <= 16 libstdc++ runs a
 // stable insertion sort, so a stable rank sort is exact in both cases; otherwise one lane runs
-// the restated introsort. Returns false, with sk/sv unchanged, when a key is NaN.
-__device__ bool sort_like_std(float* sk, int* sv, int n, float* tmpk, int* tmpv) {
+// the restated introsort.
+__device__ void sort_like_std(float* sk, int* sv, int n, float* tmpk, int* tmpv) {
   const int lane = lane_id();
-  bool tie = false, nan = false;
+  bool tie = false;
   for (int t = lane; t < n; t += 32) {
     const float kt = sk[t];
     int rank = 0;
-    nan |= !(kt == kt);
     for (int u = 0; u < n; ++u) {
       const float ku = sk[u];
       rank += (ku < kt) || (ku == kt && u < t);
@@ -248,7 +252,6 @@ __device__ bool sort_like_std(float* sk, int* sv, int n, float* tmpk, int* tmpv)
     tmpv[rank] = sv[t];
   }
   const bool anytie = __any_sync(kFull, tie);
-  if (__any_sync(kFull, nan)) return false;
   __syncwarp();
   if (!anytie || n <= 16) {
     for (int t = lane; t < n; t += 32) {
@@ -259,7 +262,6 @@ __device__ bool sort_like_std(float* sk, int* sv, int n, float* tmpk, int* tmpv)
     lib_std_sort(KV{sk, sv}, n);
   }
   __syncwarp();
-  return true;
 }
 
 // ------------------------------------------------------------------ sorted candidate array
@@ -330,8 +332,7 @@ __device__ int sorted_insert(uint2* items, int& num, int cap, float key, int id)
 // merged position is its lower bound in the array plus its rank in the batch; array items from
 // the first insertion point on move right by the number of batch keys below them (processed
 // from the tail, so nothing is overwritten before it is read). Returns false, with nothing
-// changed, when a tie exists or a batch key is NaN (the array must hold none; kInt: keys are integers).
-template <bool kInt = false>
+// changed, when a tie exists.
 __device__ bool merge_unsorted_batch(uint2* items, int& num, int cap, const float* sk, const int* sv, int m,
                                      float* tk, int* tv, int* first_pos) {
   const int lane = lane_id();
@@ -344,7 +345,6 @@ __device__ bool merge_unsorted_batch(uint2* items, int& num, int cap, const floa
     if (i >= m) break;
     const float key = sk[i];
     int rank = 0;
-    if (!kInt) tie |= !(key == key);
     for (int u = 0; u < m; ++u) {
       const float ku = sk[u];
       rank += ku < key;
@@ -408,29 +408,6 @@ __device__ bool merge_unsorted_batch(uint2* items, int& num, int cap, const floa
   __syncwarp();
   return true;
 }
-
-// Inserts an expansion's kept neighbours sk/sv[0..m) (in list order) into items[0..num): the batch merge
-// when nothing ties (*merged is then set), else std::sort's order and one insertion after another.
-// Returns the smallest insertion index. NaN keys have no place in an order: merged positions would
-// collide and leave others unwritten, so from the first NaN on (an infinite query coordinate times a
-// zero, for one) neighbours are inserted one by one as they come. `count` is turned negative (~) then:
-// a counter that the caller does not change meanwhile, as these kernels have no register to spare.
-template <bool kInt = false>
-__device__ __forceinline__ int insert_batch(uint2* items, int& num, int cap, float* sk, int* sv, int m, float* tk,
-                                            int* tv, int& count, bool* merged = nullptr) {
-  int p0;
-  if (kInt || count >= 0) {
-    if (merge_unsorted_batch<kInt>(items, num, cap, sk, sv, m, tk, tv, &p0)) {
-      if (merged) *merged = true;
-      return p0;
-    }
-    if (!sort_like_std(sk, sv, m, tk, tv) && !kInt) count = ~count;
-  }
-  p0 = 0x7fffffff;
-  for (int i = 0; i < m; ++i) p0 = min(p0, sorted_insert(items, num, cap, sk[i], sv[i]));
-  return p0;
-}
-__device__ __forceinline__ int plain_count(int count) { return count < 0 ? ~count : count; }
 
 __device__ void write_result_row(const SearchArgs& a, int64_t qi, const uint2* res, int cnt, bool node_sorted) {
   // res[0..cnt) sorted by key; order equal keys by node index (the reference orders them by

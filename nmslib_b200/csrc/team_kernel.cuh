@@ -35,8 +35,7 @@ struct TeamState {
   int tcount;              // entries of the table
   int st_dist, st_expand, st_greedy, st_list_ints;
   int overflow;
-  int ready;                 // V1Merge: how many of the first candidates in line are evaluated,
-  int nan;                   // and -1 once the array has held a NaN key, else 0
+  int line, ready;           // V1Merge: candidates in line (at most 16), how many of the first are evaluated
   int tied;                  // equal keys met where SearchOld's order among them would matter
   float edge_in, edge_out;   // SearchOld's walk: the last key that stays in the array, the first that falls off,
   float edge_tie;            // the key at the array's end that another like it fell off or was rejected at,
@@ -396,7 +395,7 @@ __device__ __forceinline__ void team_eval(const DevIndex& ix, const float* q, in
     team_dists<D, NF, R>(ix, q, id, act, d);
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (act[r] && (lane_id() & (GL - 1)) == 0) put(base + r * kGroups + group, d[r]);
+      if (act[r] && (lane_id() & (GL - 1)) == 0) put(base + r * kGroups + group, kept_dist(d[r]));
   }
 }
 
@@ -521,20 +520,21 @@ __device__ void team_result_offer(uint2* res, int& size, int k, float d, int nod
 }
 
 // ------------------------------------------------------------------ beam merge
-// Kept neighbours sk/sv[0..qty) inserted the general way (equal keys, NaN, more of them than threads).
-// Returns the smallest insertion position; st.tied is set unless the batch merge took them.
-__device__ __noinline__ int team_insert_general(TeamState& st, uint2* items, int cap, float* sk, int* sv, int qty,
-                                                float* tk, int* tv) {
-  int num = uni(st.num);
-  int nan = uni(st.nan);
-  bool merged = false;
-  const int p0 = insert_batch(items, num, cap, sk, sv, qty, tk, tv, nan, &merged);
-  __syncwarp();
-  if (lane_id() == 0) {
-    st.num = num;
-    st.nan = nan;
-    if (!merged) st.tied = 1;
+// Kept neighbours sk/sv[0..qty) inserted the general way (equal keys, more of them than threads):
+// the batch merge when nothing ties, else std::sort's order and one insertion after another. Returns
+// the smallest insertion position; *num_io is the array's size.
+__device__ __noinline__ int team_insert_general(uint2* items, int* num_io, int cap, float* sk, int* sv, int qty,
+                                                float* tk, int* tv, int* tied) {
+  const int lane = lane_id();
+  int num = *num_io, p0 = 0x7fffffff;
+  if (!merge_unsorted_batch(items, num, cap, sk, sv, qty, tk, tv, &p0)) {
+    if (lane == 0) *tied = 1;
+    sort_like_std(sk, sv, qty, tk, tv);
+    p0 = 0x7fffffff;
+    for (int i = 0; i < qty; ++i) p0 = min(p0, sorted_insert(items, num, cap, sk[i], sv[i]));
   }
+  __syncwarp();
+  if (lane == 0) *num_io = num;
   __syncwarp();
   return p0;
 }
@@ -627,7 +627,10 @@ __device__ __forceinline__ void team_line_v1(const SearchArgs& a, const TeamView
     if (!found) curr = min(t0 + 32, end);
   }
   found = min(found, 16);
-  if (lane == 0) st.curr = curr;
+  if (lane == 0) {
+    st.curr = curr;
+    st.line = found;
+  }
   __syncwarp();
   team_plan(a, v, lane >= 16 ? st.slot_node[lane - 16] : -1, lane < found ? st.line_node[lane] : -1);
   // over: SearchOld's walk, see team_expand_v1
@@ -670,7 +673,8 @@ __device__ __noinline__ void team_insert_ordered(const TeamView& v, int n, int e
       __syncwarp();
     }
     if (qty) {
-      const int p0 = team_insert_general(st, v.items(), cap, v.sk(), v.sv(), qty, v.nb_d(), v.nb_id());
+      const int p0 = team_insert_general(v.items(), &st.num, cap, v.sk(), v.sv(), qty, v.nb_d(), v.nb_id(),
+                                         &st.tied);
       if (lane == 0) st.first = min(st.first, p0);
       __syncwarp();
     }
@@ -688,7 +692,7 @@ __device__ __noinline__ void team_insert_ordered(const TeamView& v, int n, int e
 // an equal key, unless its exponential probe can meet one of several equals or the equal key is the
 // last at that moment. So a kept item lands at (array keys below it) + (kept keys below it) and an
 // array item moves right by the number of kept keys not above it. Where that may not hold (equal
-// kept keys, two equal array keys, an equal one at the array's end, any NaN, more kept than threads) the
+// kept keys, two equal array keys, an equal one at the array's end, more kept than threads) the
 // kept ones are inserted one by one in the reference's order instead.
 //
 // `old`: SearchOld (hnsw_distfunc_opt.cc:285-381) with k <= ef, which is this walk too. Its candidates
@@ -823,7 +827,6 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
     if (mine) {
       d = sk[u];
       id = v.sv()[u];
-      hard = st.nan != 0;
       int lo = 0, hi = num;
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -840,11 +843,9 @@ __device__ __forceinline__ void team_expand_v1(const SearchArgs& a, const TeamVi
       }
       if (old && equal > 1)  // in the order they were kept
         for (int w = 0; w < u; ++w) rank += sk[w] == d;
-      if (old) {
-        hard |= equal == 0;  // NaN
-      } else {
+      if (!old) {
         const bool twin = lo < num && key_of(items[lo]) == d;
-        hard |= equal != 1;  // itself; 0: NaN
+        hard = equal != 1;  // itself
         hard |= twin && (lo + 1 >= num || lo + rank + 1 >= cap || key_of(items[lo + 1 < num ? lo + 1 : lo]) == d);
       }
       pos = lo + rank;
@@ -1015,8 +1016,6 @@ __device__ __forceinline__ void team_commit_old(const SearchArgs& a, const TeamV
   __syncwarp();
   if (open && rank < 16) st.line_node[rank] = (int)c.y;
   __syncwarp();
-  if (lane == 0) st.line_node[0] = (int)c.y;  // the top comes first (NaN distances have no ranks)
-  __syncwarp();
   team_plan(a, v, slot_node, lane < 16 ? st.line_node[lane] : -1);
 }
 
@@ -1139,8 +1138,7 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
         bool fresh = false;
         const int ti = team_insert(v, (uint32_t)cur, &fresh);
         v.tkey()[ti] = (uint32_t)cur | kTabVisited;
-        st.curr = 0;
-        st.nan = curdist == curdist ? 0 : -1;
+        st.curr = st.line = 0;
         st.num = 1;
         st.tcount = 1;
         st.st_expand = 0;

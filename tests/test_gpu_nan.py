@@ -1,5 +1,6 @@
 """NaN distances (an infinite query coordinate against rows with zeros there, NaN rows, NaN queries) in every
-search kernel. NaN has no order, so no list is asked for; every result is a row of the index, once."""
+search kernel. A NaN distance counts as infinite; every result is a row of the index, once, in ascending
+order."""
 import struct
 
 import numpy as np
@@ -52,7 +53,8 @@ def test_nan_distances_stay_in_range(tmp_path, space, dim, nan_rows):
         for algo, k, ef in (("v1merge", 10, 30), ("v1merge", 10, 200), ("v1merge", 40, 20), ("old", 10, 100)):
             idx.setQueryTimeParams({"efSearch": ef, "algoType": algo})
             idx.setLaunchConfig(**shape)
-            ids, _, cnt = idx.knnQueryBatchArrays(q[:nq], k)
+            ids, d, cnt = idx.knnQueryBatchArrays(q[:nq], k)
+            assert (d[:, 1:] >= d[:, :-1]).all()
             assert (cnt >= 1).all() and (cnt <= k).all()
             live = np.arange(k) < cnt[:, None]
             assert (ids[live] >= 0).all() and (ids[live] < N).all() and (ids[~live] == -1).all()
