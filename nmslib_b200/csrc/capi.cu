@@ -195,7 +195,7 @@ static bool cap_bulk_round(const DevIndex& d, int* rows) {
 }
 
 int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bool with_old, bool plain,
-                LaunchPlan* out, std::string* err) {
+                LaunchPlan* out, std::string* err, double per_sm) {
   LaunchPlan p;
   p.with_old = with_old;
   p.nbpad = ((std::max(d.maxM, d.maxM0) + 1 + 31) / 32) * 32;
@@ -269,7 +269,9 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
     const bool bulk = cfg.row_copy != 1;
     int rows = p.stage_rows;
     // An expansion brings 9-14 new rows: 12 a round take most in one, where 8 take two row latencies and 4
-    // three or four. More rows a round cost shared memory, in two ways (10K queries, M 16 unless said, us):
+    // three or four. More rows a round cost shared memory, which counts in two ways once there are half
+    // again to twice as many queries as resident warps (10K queries, M 16 unless said, us; 200K x 128,
+    // efSearch 200, 4,500 queries: 2,009 / 1,990 / 1,935):
     //  * past some beam 12 rows lose resident blocks (1M x 128, rows per round 4 / 8 / 12: efSearch 100:
     //    2,152 / 1,993 / 1,952, 256: 3,958 / 3,887 / 4,064, 400: 5,291 / 5,283 / 6,224; 1M x 100, M 24,
     //    100: 2,244 / 2,047 / 2,168), sooner where the index lies in L2 and a row latency is short
@@ -285,12 +287,21 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
       const double index_mb = (double)d.n * row_bytes / 1e6;
       const bool short_lists = lists <= 32;
       int max12 = short_lists ? 112 : 64, max8 = short_lists ? 400 : 220;
-      if (lists > 24) {
-        if (index_mb <= 126 && (short_lists ? d.dim >= 120 : d.dim > 64)) max12 = 48;
+      if (per_sm >= 36 && lists > 24) {
+        if (per_sm >= 50 && index_mb <= 126 && (short_lists ? d.dim >= 120 : d.dim > 64)) max12 = 48;
         const int l1_kept = (196 * 1024 / 8 - 1024) / 4 - nbpad * 16 - 16 - 8 * row_bytes;  // left for the beam
         if (!(short_lists && d.dim > 96 && index_mb >= 350)) max8 = std::min(max8, l1_kept / 8);
       }
       rows = p.region <= max12 ? 12 : p.region <= max8 ? 8 : 4;
+      // a batch that fewer rows a round hold all at once would need a second turn otherwise (4,500 queries,
+      // 10K x 128: efSearch 64: 463 / 435 / 519, 400: 1,273 / 1,784 / 1,844)
+      auto resident = [&](int r) {
+        const int block = kWarpsPerBlock * lean_smem_bytes(d, p.region, nbpad, r) + 1024;
+        return kWarpsPerBlock * std::min(8, 228 * 1024 / block);
+      };
+      const int planned = rows;
+      for (int r = 8; r >= 4 && per_sm > resident(rows); r -= 4)
+        if (r < planned && per_sm <= resident(r)) rows = r;
     }
     if (bulk) cap_bulk_round(d, &rows);
     const int ws = lean_smem_bytes(d, p.region, nbpad, rows);
@@ -302,6 +313,9 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
       p.warp_smem = ws;
     }
   }
+  int least_smem = p.warp_smem;  // with the fewest rows a round that a batch of another size may take
+  if (p.lean && cfg.stage_rows == 0 && d.dim <= 128)
+    least_smem = lean_smem_bytes(d, p.region, p.nbpad, std::min(p.stage_rows, 4));
   p.wpb = plain ? 1 : (cfg.warps_per_block ? cfg.warps_per_block : kWarpsPerBlock);
   while (p.wpb > 1 && p.wpb * p.warp_smem > kMaxSmemPerBlock) p.wpb >>= 1;
   if (p.wpb * p.warp_smem > kMaxSmemPerBlock) {
@@ -316,6 +330,9 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
     *err = "no resident block fits this configuration";
     return NMSG_ERR_DEVICE;
   }
+  p.slot_blocks = p.blocks_per_sm;
+  if (least_smem < p.warp_smem)  // 228 KB an SM, a KB of it a block's own; eight lean blocks at most
+    p.slot_blocks = std::max(p.slot_blocks, std::min(8, 228 * 1024 / (p.wpb * least_smem + 1024)));
   *out = p;
   return NMSG_OK;
 }
@@ -700,7 +717,7 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
   a.kmax = kmax;
   LaunchPlan plan;
   std::string perr;
-  int rc = plan_launch(d, h->cfg, region, any_old, plain, &plan, &perr);
+  int rc = plan_launch(d, h->cfg, region, any_old, plain, &plan, &perr, (double)nq / std::max(1, h->num_sms));
   if (rc != NMSG_OK) return fail(rc, perr);
   region = plan.region;
   plan.old_share = !any_old ? 0.0 : k_per_q || ef_per_q ? (double)num_old / (double)nq : 1.0;
@@ -714,10 +731,10 @@ int knn_batch_impl(nmsg_index* h, const void* queries_v, bool u8, int64_t nq, in
                                                         : bps * h->num_sms)
                                : blocks * wpb * plan.ctx;
   if (!plain) a.team = plan_team(d, h->cfg, plan, nq, h->num_sms);
-  // visited sets: as many as the one-warp kernels have resident at this beam size, whatever the batch's
+  // visited sets: as many as the one-warp kernels can have resident at this beam size, whatever the batch's
   // size, so that growing batches do not grow them (an allocation in mid-service, refused under stream
   // capture). The team kernel rarely has more blocks; it makes do with these.
-  const int slots = warp_slots;
+  const int slots = plain ? warp_slots : std::max(warp_slots, plan.slot_blocks * h->num_sms * wpb * plan.ctx);
   a.team.blocks = std::min(a.team.blocks, slots);
   a.ctx_per_warp = plan.ctx;
   a.bulk_rows = plan.bulk_rows ? 1 : 0;

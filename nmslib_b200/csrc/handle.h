@@ -38,6 +38,7 @@ struct LaunchPlan {
   int warp_smem = 0;
   int wpb = kWarpsPerBlock;
   int blocks_per_sm = 0;
+  int slot_blocks = 0;    // blocks per SM that batches of any size can have resident with this beam
   bool with_old = false;
   double old_share = 0;   // share of the batch's queries that take SearchOld (the caller's to set)
   int ctx = 1;            // queries per persistent warp (> 1: search_multi_kernel)
@@ -46,9 +47,10 @@ struct LaunchPlan {
 };
 
 // Chooses gather mode, shared-memory sizes and warps per block for a launch whose largest query
-// needs `region` items, honouring explicit settings in cfg; returns an nmsg_status.
+// needs `region` items, honouring explicit settings in cfg; returns an nmsg_status. per_sm: the batch's
+// queries per SM, 0 when others may join it.
 int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bool with_old, bool plain,
-                LaunchPlan* out, std::string* err);
+                LaunchPlan* out, std::string* err, double per_sm = 0);
 
 // The team kernel's shape for a batch of nq queries whose largest needs `region` items, or
 // warps == 0 when the batch runs on the kernels plan_launch chose (an explicit launch shape, or
