@@ -264,7 +264,14 @@ int plan_launch(const DevIndex& d, const nmsg_launch_config& cfg, int region, bo
   // the lean kernel: V1Merge with one query per warp over the index shapes it is compiled for,
   // rows staged by one bulk copy each, or by 16-byte copies spread over the lanes (row_copy 1)
   p.lean = false;
-  if (!plain && !with_old && p.gather == 0 && p.hash_log2 == 0 && p.ctx == 1 && lean_supported(d)) {
+  // Not for wide rows with a remainder and middling long beams, where its spilled registers cost more than
+  // the general kernel's loops (10,000 queries, lean / general, us: cosine 500K x 200, M 24, efSearch 200:
+  // 4,106 / 4,538, 256: 5,398 / 5,138, 400: 7,170 / 6,520, 600: 9,533 / 9,829; l2 200K x 200, M 16, 320: 5,484 /
+  // 5,471, 400: 6,375 / 6,230; x 130, M 32, 320: 5,278 / 5,823, 400: 6,888 / 6,671; 500K x 140, M 16, never).
+  const bool long_lists = std::max(d.maxM, d.maxM0) > 32;
+  const int lean_beam = d.dim > 192 ? (long_lists ? 220 : 320) : long_lists ? 320 : 512;
+  const bool lean_slower = d.dim % 16 && d.dim > 128 && p.region > lean_beam && p.region <= 512;
+  if (!plain && !with_old && p.gather == 0 && p.hash_log2 == 0 && p.ctx == 1 && lean_supported(d) && !lean_slower) {
     const int nbpad = std::max(32, ((std::max(d.maxM, d.maxM0) + 31) / 32) * 32);
     const bool bulk = cfg.row_copy != 1;
     int rows = p.stage_rows;
