@@ -395,7 +395,8 @@ __device__ __forceinline__ void team_eval(const DevIndex& ix, const float* q, in
     team_dists<D, NF, R>(ix, q, id, act, d);
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (act[r] && (lane_id() & (GL - 1)) == 0) put(base + r * kGroups + group, kept_dist(d[r]));
+      if (act[r] && (lane_id() & (GL - 1)) == 0)  // cosine, LInf and bytes have no NaN
+        put(base + r * kGroups + group, D == kTeamL2 || D == kTeamNeg || D == kTeamL1 ? kept_dist(d[r]) : d[r]);
   }
 }
 
@@ -1117,7 +1118,7 @@ __device__ __forceinline__ void team_query(const SearchArgs& a, const TeamView& 
   }
   // ---- level 0: the entry point is visited and first in line
   const TeamHeap heap{v.heap(), OLD ? a.old_heap + (int64_t)slot * a.old_heap_cap : nullptr, a.team.heap_items};
-  // SearchOld with heaps, or (k <= ef, unless equal distances meet at the array's end) as V1Merge's walk
+  // SearchOld with heaps, or (k <= ef, unless equal distances count, see team_expand_v1) as V1Merge's walk
   bool heaps = OLD && use_old && k > ef;
   const int kth = OLD && use_old ? k : INT_MAX;
   const int walk_dist = uni(st.st_dist), walk_ints = uni(st.st_list_ints);
